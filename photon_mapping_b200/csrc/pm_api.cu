@@ -3,6 +3,8 @@
 #include "../../include/pm_cuda.h"
 #include "pm_api_internal.cuh"
 #include "pm_hostio.cuh"
+#include "pm_knn_tile.cuh"
+#include "pm_sort.cuh"
 
 #include <cstdio>
 #include <cstring>
@@ -87,9 +89,9 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
     return PM_OK;
   }
   if ((st_ok = dm.aos.ensure((size_t)n * 9 * sizeof(float))) ||
-      (st_ok = dm.pos4.ensure((size_t)n * sizeof(float4))) ||
-      (st_ok = dm.thr4.ensure((size_t)n * sizeof(float4))) ||
-      (st_ok = dm.wi2.ensure((size_t)n * sizeof(float2))) ||
+      (st_ok = dm.pos4.ensure(map_places(n) * sizeof(float4))) ||
+      (st_ok = dm.thr4.ensure(map_places(n) * sizeof(float4))) ||
+      (st_ok = dm.wi2.ensure(map_places(n) * sizeof(float2))) ||
       (st_ok = dm.boxes.ensure((size_t)total * 2 * sizeof(float4))) ||
       (st_ok = c->scratch.ensure(map_build_scratch_bytes(n))))
     return set_err(c, st_ok, "photon map allocation (%lld photons)",
@@ -108,6 +110,68 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
   if (e != cudaSuccess) return cuda_status(c, e, "photon map build");
   dm.built = true;
   return PM_OK;
+}
+
+// A scratch buffer of `bytes` for work on stream st, ordered after the work
+// that used it last (whatever stream that was on); `done` must be recorded
+// on st once the last kernel that touches the buffer is enqueued.
+static int take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st, StreamScratch** out) {
+  StreamScratch* pick = nullptr;
+  for (auto& x : c->stream_scratch) {
+    if (x.done && cudaEventQuery(x.done) != cudaSuccess) {
+      cudaGetLastError();  // still in use
+      if (x.last == st && !pick) pick = &x;
+      continue;
+    }
+    pick = &x;
+    break;
+  }
+  if (!pick) pick = &c->stream_scratch[c->scratch_next++ % kStreamScratch];
+  cudaError_t e = cudaSuccess;
+  if (!pick->done) e = cudaEventCreateWithFlags(&pick->done, cudaEventDisableTiming);
+  else e = cudaStreamWaitEvent(st, pick->done, 0);
+  if (e != cudaSuccess) return cuda_status(c, e, "query scratch");
+  // growing frees the old buffer, which waits for the device
+  if (pick->buf.ensure(bytes) != PM_OK)
+    return set_err(c, PM_ERR_OUT_OF_MEMORY, "query scratch (%zu bytes)", bytes);
+  pick->last = st;
+  *out = pick;
+  return PM_OK;
+}
+
+bool use_tiles(const pm_ctx* c, const DevMap& dm, int64_t nq, int k, bool sorted) {
+  return nq * (k + 50) >= (sorted ? kTileMinWork / 2 : kTileMinWork) && nq <= (int64_t)0x7fffffff && dm.n >= kTileMinPhotons &&
+         k <= kTileMaxK && !c->stats_on;
+}
+
+// Radiance estimates of unordered device queries on stream st: their order
+// by Morton code, then the tile kernel, then what it left.
+int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq, int k,
+                       float n_emitted, float* d_rgb, cudaStream_t st) {
+  const size_t words = 4 * (size_t)nq + sort_hist_words(nq) + 16;
+  StreamScratch* sc = nullptr;
+  int s = take_scratch(c, words * 4, st, &sc);
+  if (s != PM_OK) return s;
+  uint32_t* ka = (uint32_t*)sc->buf.ptr;
+  uint32_t* kb = ka + nq;
+  uint32_t* va = kb + nq;
+  uint32_t* vb = va + nq;
+  uint32_t* hist = vb + nq;
+  const MapDev m = map_view(dm);
+  query_keys_launch(m, d_q, nq, 3, ka, va, st);
+  const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, (int)nq, kQueryKeyBits, hist, st);
+  // the keys' place is free again: the list of the queries left
+  const TileDefer left{ka, hist, false};
+  cudaError_t e = knn_tile_launch(m, d_q, nq, k, n_emitted, d_rgb, left, c->next_counter(),
+                                  c->num_sms, st, in_b ? vb : va, 3);
+  if (e == cudaSuccess) {
+    KnnOut o{};
+    o.rgb = d_rgb;
+    e = knn_launch(m, d_q, nq, k, kModeRadiance, n_emitted, o, c->next_counter(), c->num_sms, st,
+                   ka, 3, hist);
+  }
+  const cudaError_t e2 = cudaEventRecord(sc->done, st);
+  return cuda_status(c, e != cudaSuccess ? e : e2, "radiance launch");
 }
 
 }  // namespace pm
@@ -368,6 +432,11 @@ int pm_photonmap_radiance(pm_ctx* c, int map, const pm_radiance_query* q,
   if (d_q && ((uintptr_t)d_q & 15) != 0) d_q = nullptr;
   // a mapped output buffer is written by the kernel itself
   float* mapped_out = (float*)mapped_host(out_rgb);
+  // the tile kernel reads and writes records in another order than the
+  // caller's, which host memory serves badly: queries and output are staged
+  // on the device and stream through the mapping whole
+  const bool tiles = use_tiles(c, dm, nq, k, false);
+  if (tiles) d_q = mapped_out = nullptr;
   int s = PM_OK;
   if ((!d_q && (s = c->q_in.ensure(qb))) || (!mapped_out && (s = c->q_out.ensure(ob))))
     return set_err(c, s, "query buffers");
@@ -379,11 +448,16 @@ int pm_photonmap_radiance(pm_ctx* c, int map, const pm_radiance_query* q,
   KnnOut o{};
   o.stats = c->stats_ptr();
   o.rgb = mapped_out ? mapped_out : (float*)c->q_out.ptr;
-  e = knn_launch(map_view(dm), d_q, nq, k, kModeRadiance,
-                 (float)n_emitted, o, c->next_counter(), c->num_sms, st);
-  if (e != cudaSuccess) return cuda_status(c, e, "radiance launch");
+  if (tiles) {
+    if ((s = radiance_unordered(c, dm, d_q, nq, k, (float)n_emitted, o.rgb, st)) != PM_OK)
+      return s;
+  } else {
+    e = knn_launch(map_view(dm), d_q, nq, k, kModeRadiance,
+                   (float)n_emitted, o, c->next_counter(), c->num_sms, st);
+    if (e != cudaSuccess) return cuda_status(c, e, "radiance launch");
+  }
   if (!mapped_out) {
-    e = cudaMemcpyAsync(out_rgb, o.rgb, ob, cudaMemcpyDeviceToHost, st);
+    e = copy_out(out_rgb, o.rgb, ob, c->num_sms, st);
     if (e != cudaSuccess) return cuda_status(c, e, "radiance download");
   }
   return cuda_status(c, cudaStreamSynchronize(st), "radiance");
@@ -406,6 +480,14 @@ int pm_photonmap_radiance_device(pm_ctx* c, int map, const void* d_queries,
   cudaSetDevice(c->device);
   DevMap& dm = c->maps[map];
   if (!dm.built) return set_err(c, PM_ERR_NOT_BUILT, "map %d not built", map);
+  // a captured launch keeps no buffer of the context: it takes the
+  // warp-per-query kernel, which needs none
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (use_tiles(c, dm, nq, k, false) &&
+      cudaStreamIsCapturing(as_stream(stream), &cap) == cudaSuccess &&
+      cap == cudaStreamCaptureStatusNone)
+    return radiance_unordered(c, dm, d_queries, nq, k, (float)n_emitted, (float*)d_out_rgb,
+                              as_stream(stream));
   KnnOut o{};
   o.stats = c->stats_ptr();
   o.rgb = (float*)d_out_rgb;

@@ -48,7 +48,7 @@ struct pm_batch {
     int lvl_cnt[kMaxLevels] = {};
   };
   std::vector<Shape> shape;
-  std::vector<int64_t> box_base;
+  std::vector<int64_t> box_base, group_off;
   DevBuf m_pos4, m_thr4, m_wi2, m_boxes, m_keys_b, m_va, m_vb, m_hist, m_bb, m_tab, m_lvl;
   DevBuf m_order, m_count, m_first, m_sums;
   BatchMapBuild mb{};
@@ -141,9 +141,11 @@ int upload_tables(pm_batch* b) {
     a.err = errw;
     MapDev& mv = x.map;
     const pm_batch::Shape& sh = b->shape.empty() ? pm_batch::Shape{} : b->shape[s];
-    mv.pos4 = (const float4*)b->m_pos4.ptr + b->cap_off[s];
-    mv.thr4 = (const float4*)b->m_thr4.ptr + b->cap_off[s];
-    mv.wi2 = (const float2*)b->m_wi2.ptr + b->cap_off[s];
+    const size_t place0 =
+        b->group_off.empty() ? 0 : (size_t)(b->group_off[s] + s) * kGroup;
+    mv.pos4 = (const float4*)b->m_pos4.ptr + place0;
+    mv.thr4 = (const float4*)b->m_thr4.ptr + place0;
+    mv.wi2 = (const float2*)b->m_wi2.ptr + place0;
     mv.boxes = b->box_base.empty() ? nullptr : (const float4*)b->m_boxes.ptr + 2 * b->box_base[s];
     mv.n = b->shape.empty() ? 0 : (int)b->stored[s];
     mv.nlevels = sh.nlevels;
@@ -241,7 +243,9 @@ int plan_maps(pm_batch* b) {
                 (long long)total);
   b->shape.assign((size_t)n, pm_batch::Shape{});
   b->box_base.assign((size_t)n + 1, 0);
-  std::vector<int64_t> group_off((size_t)n + 1, 0), level_off((size_t)kMaxLevels * (n + 1), 0);
+  std::vector<int64_t>& group_off = b->group_off;
+  group_off.assign((size_t)n + 1, 0);
+  std::vector<int64_t> level_off((size_t)kMaxLevels * (n + 1), 0);
   std::vector<int> lvl((size_t)n * 2 * kMaxLevels, 0);
   int max_levels = 0;
   for (int s = 0; s < n; ++s) {
@@ -259,6 +263,8 @@ int plan_maps(pm_batch* b) {
   }
   const size_t tn = (size_t)std::max<int64_t>(total, 1);
   const size_t nb = (size_t)std::max<int64_t>(b->box_base[n], 1);
+  // one group without photons per scene
+  const size_t places = (size_t)(group_off[n] + n) * kGroup;
   std::vector<int64_t> tab;
   tab.insert(tab.end(), b->cap_off.begin(), b->cap_off.end());
   tab.insert(tab.end(), group_off.begin(), group_off.end());
@@ -267,8 +273,8 @@ int plan_maps(pm_batch* b) {
   tab.insert(tab.end(), b->emit_off.begin(), b->emit_off.end());
   const size_t te = (size_t)std::max<int64_t>(b->total_emit, 1);
   int s;
-  if ((s = b->m_pos4.ensure(tn * 16)) || (s = b->m_thr4.ensure(tn * 16)) ||
-      (s = b->m_wi2.ensure(tn * 8)) || (s = b->m_boxes.ensure(nb * 32)) ||
+  if ((s = b->m_pos4.ensure(places * 16)) || (s = b->m_thr4.ensure(places * 16)) ||
+      (s = b->m_wi2.ensure(places * 8)) || (s = b->m_boxes.ensure(nb * 32)) ||
       (s = b->m_keys_b.ensure(tn * 8)) || (s = b->m_va.ensure(tn * 4)) ||
       (s = b->m_vb.ensure(tn * 4)) || (s = b->m_order.ensure(tn * 4)) ||
       (s = b->m_count.ensure(te * 4)) || (s = b->m_first.ensure(te * 4)) ||

@@ -67,8 +67,8 @@ void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int
 // records [stored_off[s], stored_off[s + 1]) of raw / keys_a, and the store
 // count of the photon with work index emit_off[s] + p to count. order
 // receives, for each scene's index-order places (at the same offsets), the
-// trace record there; the map goes to pos4 / thr4 / wi2 at the same
-// offsets and the boxes from box 2 * box_base[s] on. All device arrays.
+// trace record there; scene s's map goes to pos4 / thr4 / wi2 from group
+// group_off[s] + s on (its groups and the one without photons) and the boxes from box 2 * box_base[s] on. All device arrays.
 struct BatchMapBuild {
   const float* raw;                 // total records of 9 floats
   unsigned long long* keys_a;       // total: the trace's keys, then sort scratch

@@ -141,26 +141,29 @@ __global__ void __launch_bounds__(kSegThreads)
   }
 }
 
-// Map position j of the batch: perm[j] = index-order place c, whose trace
-// record is order[c]; its index within the scene goes into pos4.w
-// (gather_kernel per scene).
+// Place t of the batch's maps (scene s's start at group group_off[s] + s):
+// perm gives the index-order place of its photon, order the trace record
+// there; the index within the scene goes into pos4.w (gather_kernel per
+// scene). Places past a scene's photons are padding.
 __global__ void __launch_bounds__(kSegThreads)
     seg_gather_kernel(const float* __restrict__ raw, const uint32_t* __restrict__ order,
-                      const uint32_t* __restrict__ perm, int64_t total,
-                      const int64_t* __restrict__ stored_off, int n, float4* __restrict__ pos4,
+                      const uint32_t* __restrict__ perm, int64_t places,
+                      const int64_t* __restrict__ stored_off,
+                      const int64_t* __restrict__ group_off, int n, float4* __restrict__ pos4,
                       float4* __restrict__ thr4, float2* __restrict__ wi2) {
   __shared__ int64_t off[kMaxBatchScenes + 1];
+  __shared__ int64_t poff[kMaxBatchScenes + 1];  // first place of each scene
   batch_load_offsets(off, stored_off, n);
+  for (int i = threadIdx.x; i <= n; i += blockDim.x) poff[i] = (group_off[i] + i) * kGroup;
   __syncthreads();
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < total;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    const int s = batch_find(off, n, j);
-    const uint32_t c = perm[j];
-    const uint32_t i = (uint32_t)(c - off[s]);
-    const float* r = raw + 9 * (size_t)order[c];
-    pos4[j] = make_float4(r[3], r[4], r[5], __uint_as_float(i));
-    thr4[j] = make_float4(r[0], r[1], r[2], r[6]);
-    wi2[j] = make_float2(r[7], r[8]);
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < places;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int s = batch_find(poff, n, t);
+    const int64_t j = off[s] + (t - poff[s]);
+    const bool in = j < off[s + 1];
+    const uint32_t c = in ? perm[j] : 0u;
+    map_store(pos4, thr4, wi2, (size_t)t, in ? raw + 9 * (size_t)order[c] : nullptr,
+              in ? (uint32_t)(c - off[s]) : 0xffffffffu);
   }
 }
 
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(kSegThreads)
     lg = g - goff[s];
     const int64_t li = lg * kGroup + (t & 7);
     if (li < stored_off[s + 1] - stored_off[s]) {
-      const float4 p = pos4[stored_off[s] + li];
+      const float4 p = pos4[(group_off[s] + s) * kGroup + li];
       lo.x = fminf(lo.x, p.x); lo.y = fminf(lo.y, p.y); lo.z = fminf(lo.z, p.z);
       hi.x = fmaxf(hi.x, p.x); hi.y = fmaxf(hi.y, p.y); hi.z = fmaxf(hi.z, p.z);
     }
@@ -278,7 +281,6 @@ void batch_maps_launch(const BatchMapBuild& a, cudaStream_t st) {
   if (total <= 0) return;
   const int n = a.n_scenes;
   const int tb = kSegThreads;
-  const unsigned gb = grid_for(total, tb, a.num_sms);
   // 1. index-order places and the scenes' boxes
   exclusive_scan_u32(a.count, a.first, a.total_emit, a.sums, st);
   cudaMemsetAsync(a.bb, 0xff, 3 * sizeof(uint32_t) * (size_t)n, st);
@@ -298,8 +300,9 @@ void batch_maps_launch(const BatchMapBuild& a, cudaStream_t st) {
       a.keys_b, a.va, a.keys_a, a.vb, (int)total, 30 + a.scene_bits, a.hist, st);
   const uint32_t* perm = in_second ? a.vb : a.va;
   // 3. the map arrays
-  seg_gather_kernel<<<gb, tb, 0, st>>>(a.raw, a.order, perm, total, a.stored_off, n, a.pos4,
-                                       a.thr4, a.wi2);
+  const int64_t places = (a.total_groups + n) * kGroup;
+  seg_gather_kernel<<<grid_for(places, tb, a.num_sms), tb, 0, st>>>(
+      a.raw, a.order, perm, places, a.stored_off, a.group_off, n, a.pos4, a.thr4, a.wi2);
   // 4. the box tree, level by level
   if (a.total_groups > 0)
     seg_group_box_kernel<<<(unsigned)((a.total_groups * kGroup + tb - 1) / tb), tb, 0, st>>>(

@@ -52,4 +52,18 @@ cudaError_t copy_in(void* dst, const void* host, size_t bytes, int num_sms, cuda
   return cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, st);
 }
 
+cudaError_t copy_out(void* host, const void* src, size_t bytes, int num_sms, cudaStream_t st) {
+  if (bytes == 0) return cudaSuccess;
+  void* dst = const_cast<void*>(mapped_host(host));
+  if (dst && bytes % 16 == 0 && ((uintptr_t)src & 15) == 0 && ((uintptr_t)dst & 15) == 0) {
+    const size_t n16 = bytes / 16;
+    size_t blocks = (n16 + 255) / 256;
+    const size_t cap = (size_t)num_sms * 8;
+    if (blocks > cap) blocks = cap;
+    stream_copy_kernel<<<(unsigned)blocks, 256, 0, st>>>((uint4*)dst, (const uint4*)src, n16);
+    return cudaGetLastError();
+  }
+  return cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, st);
+}
+
 }  // namespace pm

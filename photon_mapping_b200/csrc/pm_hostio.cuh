@@ -15,4 +15,8 @@ const void* mapped_host(const void* p);
 // cudaMemcpyAsync otherwise.
 cudaError_t copy_in(void* dst, const void* host, size_t bytes, int num_sms, cudaStream_t st);
 
+
+// Device -> host copy on st (the same rule as copy_in).
+cudaError_t copy_out(void* host, const void* src, size_t bytes, int num_sms, cudaStream_t st);
+
 }  // namespace pm

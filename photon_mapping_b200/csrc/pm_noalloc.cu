@@ -42,9 +42,9 @@ constexpr size_t noalloc_boxes(size_t n) {
   return total;
 }
 
-constexpr size_t kNaPos4 = align256((size_t)kNoAllocMaxPhotons * 16);
-constexpr size_t kNaThr4 = align256((size_t)kNoAllocMaxPhotons * 16);
-constexpr size_t kNaWi2 = align256((size_t)kNoAllocMaxPhotons * 8);
+constexpr size_t kNaPos4 = align256(map_places(kNoAllocMaxPhotons) * 16);
+constexpr size_t kNaThr4 = align256(map_places(kNoAllocMaxPhotons) * 16);
+constexpr size_t kNaWi2 = align256(map_places(kNoAllocMaxPhotons) * 8);
 constexpr size_t kNaBoxes = align256(noalloc_boxes(kNoAllocMaxPhotons) * 32);
 // map_build_scratch_bytes(n): keys/values a/b, tile histogram, box words
 constexpr size_t kNaSort =

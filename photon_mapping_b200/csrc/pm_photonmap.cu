@@ -11,6 +11,7 @@
 //   integrator.h:133-152  radiance estimate with the Lambert BRDF
 //   material.h:80-88      Lambert::evaluate
 #include "pm_batch.cuh"
+#include "pm_knn_tile.cuh"
 #include "pm_photonmap.cuh"
 #include "pm_sort.cuh"
 
@@ -96,18 +97,16 @@ __global__ void morton_kernel(const float* __restrict__ aos, int n,
   vals[i] = (uint32_t)i;
 }
 
-__global__ void gather_kernel(const float* __restrict__ aos, int n,
+// Place t of the map from its photon's record (places past n: padding).
+__global__ void gather_kernel(const float* __restrict__ aos, int n, int places,
                               const uint32_t* __restrict__ order,
                               float4* __restrict__ pos4,
                               float4* __restrict__ thr4,
                               float2* __restrict__ wi2) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t i = order[s];
-  const float* r = aos + 9 * (size_t)i;
-  pos4[s] = make_float4(r[3], r[4], r[5], __uint_as_float(i));
-  thr4[s] = make_float4(r[0], r[1], r[2], r[6]);
-  wi2[s] = make_float2(r[7], r[8]);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= places) return;
+  const uint32_t i = t < n ? order[t] : 0xffffffffu;
+  map_store(pos4, thr4, wi2, (size_t)t, t < n ? aos + 9 * (size_t)i : nullptr, i);
 }
 
 // Box of each 8-photon group: 8 lanes per group, 4 groups per warp.
@@ -185,7 +184,9 @@ void map_build_launch(const float* aos, int n, float4* pos4, float4* thr4,
   bbox_kernel<<<min(gb, 1184), tb, 0, st>>>(aos, n, bb);
   morton_kernel<<<gb, tb, 0, st>>>(aos, n, bb, ka, va);
   const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, n, 30, hist, st);
-  gather_kernel<<<gb, tb, 0, st>>>(aos, n, in_b ? vb : va, pos4, thr4, wi2);
+  const int places = (int)map_places(n);
+  gather_kernel<<<(places + tb - 1) / tb, tb, 0, st>>>(aos, n, places, in_b ? vb : va, pos4, thr4,
+                                                       wi2);
   const int ngroups = lvl_cnt[0];
   group_box_kernel<<<(int)(((int64_t)ngroups * kGroup + tb - 1) / tb), tb, 0,
                      st>>>(pos4, n, ngroups, boxes);
@@ -443,7 +444,7 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
   uint32_t kk, nb;
   const int bin = (int)hist_find(s.hist, (uint32_t)k, lane, &kk, &nb);
   if (nb > 32) return false;
-  int pos = 0;
+  int at = 0;
   for (int base = 0; base < cnt; base += 32) {
     const int i = base + lane;
     bool in = false;
@@ -451,8 +452,8 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
       in = min(255, __float2int_rz(__fmul_rz(__uint_as_float(s.key[i]), sc))) ==
            bin;
     const unsigned bal = __ballot_sync(kFull, in);
-    if (in) s.sel[pos + __popc(bal & lt_mask(lane))] = (uint32_t)i;
-    pos += __popc(bal);
+    if (in) s.sel[at + __popc(bal & lt_mask(lane))] = (uint32_t)i;
+    at += __popc(bal);
   }
   __syncwarp();
   uint32_t kj = 0xffffffffu, oj = 0xffffffffu;
@@ -541,6 +542,62 @@ __device__ __forceinline__ int compact_kept(const float4* pos4, WarpBuf<C>& s,
   }
   __syncwarp();
   return dst;
+}
+
+// Throughput summed over the nk kept photons listed in s.id (in the walk's
+// order) whose direction has a cosine with ns that is not negative
+// (Lambert::evaluate, material.h:80-88). Photon i of the map belongs to class
+// i & 31; a lane sums its class in list order, then the 32 classes are added
+// in a fixed tree, so the sum depends on the kept photons alone: the tile
+// kernel (pm_knn_tile.cu) adds in the same order. The photons of each class
+// are queued in s.key (its distances are no longer needed), C / 32 per class;
+// should a class need more, its lane reads the whole list instead.
+template <int C>
+__device__ __forceinline__ float3 kept_sum(const MapDev& m, WarpBuf<C>& s, int nk, float3 ns,
+                                           int lane) {
+  constexpr int kRows = C / 32;
+  uint32_t* const queue = s.key;
+  uint32_t* const count = s.hist;
+  count[lane] = 0;
+  __syncwarp();
+  for (int b = 0; b < nk; b += 32) {
+    const bool in = b + lane < nk;
+    const uint32_t id = in ? s.id[b + lane] : 0u;
+    const uint32_t c = in ? id & 31u : 32u;
+    const unsigned peers = __match_any_sync(kFull, c);
+    const uint32_t before = in ? count[c] : 0u;
+    const uint32_t r = before + __popc(peers & lt_mask(lane));
+    __syncwarp();
+    if (in && r < kRows) queue[r * 32 + c] = id;
+    if (in && (peers >> lane) == 1u) count[c] = r + 1;  // the class's last peer
+    __syncwarp();
+  }
+  const int n = (int)count[lane];
+  float x = 0.f, y = 0.f, z = 0.f;
+  auto add = [&](uint32_t id) {
+    const float4 t = __ldg(m.thr4 + id);
+    const float2 w = __ldg(m.wi2 + id);
+    if (!(dot_ref(t.w, w.x, w.y, ns.x, ns.y, ns.z) < 0.f)) {
+      x = __fadd_rn(x, t.x);
+      y = __fadd_rn(y, t.y);
+      z = __fadd_rn(z, t.z);
+    }
+  };
+  if (n <= kRows) {
+    for (int r = 0; r < n; ++r) add(queue[r * 32 + lane]);
+  } else {
+    for (int i = 0; i < nk; ++i)
+      if ((s.id[i] & 31u) == (uint32_t)lane) add(s.id[i]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {  // groups, then photons of a group
+    const int o = i == 0 ? 8 : i == 1 ? 16 : i == 2 ? 1 : i == 3 ? 2 : 4;
+    x = __fadd_rn(x, __shfl_xor_sync(kFull, x, o));
+    y = __fadd_rn(y, __shfl_xor_sync(kFull, y, o));
+    z = __fadd_rn(z, __shfl_xor_sync(kFull, z, o));
+  }
+  return make_float3(x, y, z);
 }
 
 // Per-query state of the search.
@@ -751,7 +808,8 @@ __device__ __forceinline__ float cold_tau(const float4* pos4, const float4* boxe
 // r_hint: the last exact k-th distance this warp found (in/out).
 // HIO (the single-map kernel, whose queries and output may be mapped host
 // memory): radiance records are prefetched one query ahead with cp.async,
-// and without `order` the radiance goes out in aligned groups of 8 queries.
+// and without `order` the radiance goes out in aligned groups of 8 queries
+// (`grouped`: qb is a multiple of 8; otherwise it goes out query by query).
 // Without HIO (the batched kernel, device-resident slots) records are read
 // with plain loads: measured on the 64-scene batch, the prefetch and the
 // staging code together cost it 13 % through register allocation.
@@ -760,7 +818,7 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
                                           int lane, const void* __restrict__ queries,
                                           int64_t qb, int64_t qe, int k, float n_emitted,
                                           const KnnOut& out, const uint32_t* __restrict__ order,
-                                          int stride4, float& r_hint) {
+                                          int stride4, float& r_hint, bool grouped = true) {
   const float kInf = __int_as_float(0x7f800000);
   bool have_prev = false;
   float pqx = 0.f, pqy = 0.f, pqz = 0.f, pkth = 0.f;
@@ -824,20 +882,21 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
         }
       }
       // Guess and verify when no bound is known: collect with a radius a
-      // little above the last k-th distance this warp found; k photons or
-      // more inside it make the result exact, otherwise the radius
-      // doubles (twice), then the patch bound of cold_tau is used.
+      // little above the last k-th distance this warp found, or (its first
+      // query) the radius that k photons spread evenly over the map's box
+      // faces would take; k photons or more inside it make the result exact,
+      // otherwise the radius grows by what the count suggests. The patch
+      // bound of cold_tau is the last resort: its patch may lie across the
+      // map (a query's cold start took 168k instructions in a 3.26M-photon
+      // map, where a guess takes about 4k).
       bool guess = false, need_cold = false;
-      float rg = 0.f;
+      float tg = 0.f;
       if (!warm) {
         stat_add<S>(s, lane, kStatCold, 1);
-        if (r_hint > 0.f) {
-          guess = true;
-          rg = 1.3f * r_hint;
-          q.tau = fmaxf(rg * rg, 1e-37f);
-        } else {
-          need_cold = true;
-        }
+        guess = true;
+        tg = r_hint > 0.f ? 1.69f * r_hint * r_hint : even_tau(m, L.oc[m.nlevels - 1].x, k);
+        if (!(tg > 1e-37f)) tg = 1e-37f;  // NaN too
+        q.tau = tg;
       }
       for (int attempt = 0;; ++attempt) {
         if (need_cold) {
@@ -854,9 +913,10 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
           continue;
         }
         if (!guess || q.cnt >= k) break;
-        if (attempt < 2) {
-          rg *= 2.0f;
-          q.tau = fmaxf(rg * rg, 1e-37f);
+        if (attempt < 4) {
+          // on surfaces the count grows about as the squared radius
+          tg *= fminf(1.4f * (float)k / (float)max(q.cnt, 1), 16.f);
+          q.tau = tg;
         } else {
           need_cold = true;
         }
@@ -912,52 +972,21 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       const float4 r1 = HIO ? s.rec[buf][1] : __ldg(q4 + 1);
       const float4 r2 = HIO ? s.rec[buf][2] : __ldg(q4 + 2);
       const float cos_o = dot_ref(r1.x, r1.y, r1.z, r2.x, r2.y, r2.z);
-      const float fr = __fdiv_rn(r0.w, kPI);
-      const float fg = __fdiv_rn(r1.w, kPI);
-      const float fb = __fdiv_rn(r2.w, kPI);
-      // the kept entries, in the walk's order whatever the bound was, so
-      // the sum below does not depend on the order queries are answered
       const int nk = all ? cnt : compact_kept(m.pos4, s, cnt, kth_key, kth_oid, lane);
-      float lr = 0.f, lg = 0.f, lb = 0.f;
-      for (int i = lane; i < nk; i += 32) {
-        const uint32_t id = s.id[i];
-        {
-          const float4 t = __ldg(m.thr4 + id);
-          const float2 w = __ldg(m.wi2 + id);
-          const float cos_i = dot_ref(t.w, w.x, w.y, r2.x, r2.y, r2.z);
-          // Lambert::evaluate returns 0 when either cosine is < 0
-          if (!(cos_o < 0.f) && !(cos_i < 0.f)) {
-            lr = __fadd_rn(lr, __fmul_rn(fr, t.x));
-            lg = __fadd_rn(lg, __fmul_rn(fg, t.y));
-            lb = __fadd_rn(lb, __fmul_rn(fb, t.z));
-          }
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        lr = __fadd_rn(lr, __shfl_xor_sync(kFull, lr, o));
-        lg = __fadd_rn(lg, __shfl_xor_sync(kFull, lg, o));
-        lb = __fadd_rn(lb, __shfl_xor_sync(kFull, lb, o));
-      }
-      if (lane == 0) {
-        float3 o3 = make_float3(0.f, 0.f, 0.f);
-        if (kept > 0) {
-          const float den = __fmul_rn(__fmul_rn(n_emitted, kPI), maxd2);
-          o3 = make_float3(__fdiv_rn(lr, den), __fdiv_rn(lg, den),
-                           __fdiv_rn(lb, den));
-        }
-        if (HIO && !order) {
-          float* r = reinterpret_cast<float*>(s.id + C - kStageWords) + 3 * (qi & 7);
-          r[0] = o3.x; r[1] = o3.y; r[2] = o3.z;
-        } else {
-          out.rgb[3 * rec + 0] = o3.x;
-          out.rgb[3 * rec + 1] = o3.y;
-          out.rgb[3 * rec + 2] = o3.z;
-        }
+      const float3 sum = kept_sum(m, s, nk, make_float3(r2.x, r2.y, r2.z), lane);
+      if (lane < 3) {  // a lane per channel
+        const float o = kept > 0 ? radiance_from_sum(lane == 0 ? sum.x : lane == 1 ? sum.y : sum.z,
+                                                     lane == 0 ? r0.w : lane == 1 ? r1.w : r2.w,
+                                                     cos_o, n_emitted, maxd2)
+                                 : 0.f;
+        if (HIO && !order && grouped)
+          reinterpret_cast<float*>(s.id + C - kStageWords)[3 * (qi & 7) + lane] = o;
+        else
+          out.rgb[3 * rec + lane] = o;
       }
       // work items without `order` start at multiples of 8: a group of 8 is
       // complete at qi % 8 == 7 or cut by the end of the queries
-      if (HIO && !order && ((qi & 7) == 7 || qi + 1 == qe)) {
+      if (HIO && !order && grouped && ((qi & 7) == 7 || qi + 1 == qe)) {
         __syncwarp();
         const int64_t g0 = qi & ~(int64_t)7;
         const int nf = 3 * (int)(qi + 1 - g0);
@@ -1010,7 +1039,18 @@ __global__ void __launch_bounds__(256, 4)
     knn_kernel(MapDev m, const void* __restrict__ queries, int64_t nq, int k,
                float n_emitted, KnnOut out,
                unsigned long long* __restrict__ counter,
-               const uint32_t* __restrict__ order, int stride4, int64_t head_items) {
+               const uint32_t* __restrict__ order, int stride4,
+               const uint32_t* __restrict__ nq_dev) {
+  if (nq_dev) {
+    nq = (int64_t)*nq_dev;
+    if (nq == 0) return;
+  }
+  // few queries: shorter items, so that every resident warp gets one (a query
+  // alone takes long: one warp's tree walk has no other work to hide behind)
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int tail = nq >= 8 * warps ? kTail : nq >= 4 * warps ? 4 : nq >= 2 * warps ? 2 : 1;
+  const int64_t tail_q = warps * kTail * kTailItems;
+  const int64_t head_items = nq > tail_q ? (nq - tail_q) / kChunk : 0;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Levels L;
   WarpBuf<C>& s = reinterpret_cast<WarpBuf<C>*>(smem_raw)[threadIdx.x >> 5];
@@ -1031,12 +1071,12 @@ __global__ void __launch_bounds__(256, 4)
     c0 = __shfl_sync(kFull, c0, 0);
     const int64_t item = (int64_t)c0;  // items [0, head_items) hold kChunk queries
     const bool head = item < head_items;
-    const int64_t qb = head ? item * kChunk : head_items * kChunk + (item - head_items) * kTail;
+    const int64_t qb = head ? item * kChunk : head_items * kChunk + (item - head_items) * tail;
     if (qb >= nq) break;
-    const int64_t qe = min(nq, qb + (head ? kChunk : kTail));
+    const int64_t qe = min(nq, qb + (head ? kChunk : tail));
 
     knn_chunk<C, MODE, S, true>(m, L, s, lane, queries, qb, qe, k, n_emitted, out, order, stride4,
-                          r_hint);
+                                r_hint, tail == kTail);
     if (S) {
       __syncwarp();
       if (lane < kNumStats) {
@@ -1053,7 +1093,7 @@ static cudaError_t launch_one(const MapDev& m, const void* queries,
                               int64_t nq, int k, float n_emitted, KnnOut out,
                               unsigned long long* counter, int num_sms,
                               cudaStream_t st, const uint32_t* order,
-                              int stride4) {
+                              int stride4, const uint32_t* nq_dev) {
   constexpr int kThreads = (C <= 512) ? 256 : 128;
   const size_t smem = (kThreads / 32) * sizeof(WarpBuf<C>);
   auto kern = out.stats ? knn_kernel<C, MODE, true> : knn_kernel<C, MODE, false>;
@@ -1065,44 +1105,42 @@ static cudaError_t launch_one(const MapDev& m, const void* queries,
                                                     smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  const int64_t chunks = (nq + kTail - 1) / kTail;
   const int64_t warps_per_block = kThreads / 32;
   int64_t blocks = (int64_t)num_sms * per_sm;
-  const int64_t need = (chunks + warps_per_block - 1) / warps_per_block;
+  const int64_t need = (nq + warps_per_block - 1) / warps_per_block;
   if (blocks > need) blocks = need;
   if (blocks < 1) blocks = 1;
-  const int64_t tail = blocks * warps_per_block * kTail * kTailItems;
-  const int64_t head_items = nq > tail ? (nq - tail) / kChunk : 0;
   e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)blocks, kThreads, smem, st>>>(m, queries, nq, k, n_emitted,
-                                                 out, counter, order, stride4, head_items);
+                                                 out, counter, order, stride4, nq_dev);
   return cudaGetLastError();
 }
 
 cudaError_t knn_launch(const MapDev& m, const void* queries, int64_t nq,
                        int k, int mode, float n_emitted, KnnOut out,
                        unsigned long long* counter, int num_sms,
-                       cudaStream_t st, const uint32_t* order, int stride4) {
+                       cudaStream_t st, const uint32_t* order, int stride4,
+                       const uint32_t* nq_dev) {
   if (nq <= 0) return cudaSuccess;
   if (mode == kModeAdjoint) {
     return k <= 224 ? launch_one<512, kModeAdjoint>(m, queries, nq, k, n_emitted, out, counter,
-                                                   num_sms, st, order, stride4)
+                                                   num_sms, st, order, stride4, nq_dev)
                     : launch_one<2048, kModeAdjoint>(m, queries, nq, k, n_emitted, out, counter,
-                                                    num_sms, st, order, stride4);
+                                                    num_sms, st, order, stride4, nq_dev);
   }
   if (k <= 224) {
     return mode == kModeRadiance
                ? launch_one<512, kModeRadiance>(m, queries, nq, k, n_emitted,
-                                                out, counter, num_sms, st, order, stride4)
+                                                out, counter, num_sms, st, order, stride4, nq_dev)
                : launch_one<512, kModeKnn>(m, queries, nq, k, n_emitted, out,
-                                           counter, num_sms, st, order, stride4);
+                                           counter, num_sms, st, order, stride4, nq_dev);
   }
   return mode == kModeRadiance
              ? launch_one<2048, kModeRadiance>(m, queries, nq, k, n_emitted,
-                                               out, counter, num_sms, st, order, stride4)
+                                               out, counter, num_sms, st, order, stride4, nq_dev)
              : launch_one<2048, kModeKnn>(m, queries, nq, k, n_emitted, out,
-                                          counter, num_sms, st, order, stride4);
+                                          counter, num_sms, st, order, stride4, nq_dev);
 }
 
 }  // namespace pm
