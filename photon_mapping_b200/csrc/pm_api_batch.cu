@@ -18,6 +18,7 @@
 #include "../../include/pm_cuda.h"
 #include "pm_api_internal.cuh"
 #include "pm_batch.cuh"
+#include "pm_knn_tile.cuh"
 #include "pm_scene_build.cuh"
 #include "pm_sort.cuh"
 #include "pm_trace.cuh"
@@ -56,6 +57,8 @@ struct pm_batch {
   int max_k = 1;
   pm_batch_tuning tune{8, 32, 512, 64, 128, 0};
   int knn_per_sm = 1;
+  bool tiles = false;  // the estimates by tiles of sorted queries
+  int tile_per_sm = 1;
   bool sorted_in_b = false;  // where the last query sort left its output
   cudaGraphExec_t exec = nullptr;
   BatchTables tables{};
@@ -349,16 +352,32 @@ const unsigned long long* sorted_keys(const pm_batch* b) {
   return (const unsigned long long*)(b->sorted_in_b ? b->qkb.ptr : b->qka.ptr);
 }
 
+// The estimates: by tiles where enough queries pay for them, then (or instead)
+// by the warp-per-query kernel with the tuning's launch shape.
 cudaError_t enqueue_knn(pm_batch* b, const uint32_t* order, const pm_batch_tuning& t,
                         int per_sm) {
-  batch_query_ranges_launch(sorted_keys(b), b->nq, (const unsigned*)b->qcount.ptr, b->n,
-                            t.knn_chunk, (int64_t*)b->qstart.ptr, (int64_t*)b->qoff.ptr,
+  const int chunk = b->tiles ? batch_tile_item(b->nq, b->num_sms) : t.knn_chunk;
+  batch_query_ranges_launch(sorted_keys(b), b->nq, (const unsigned*)b->qcount.ptr, b->n, chunk,
+                            (int64_t*)b->qstart.ptr, (int64_t*)b->qoff.ptr,
                             (int64_t*)b->item_off.ptr, b->st);
-  const int64_t max_items = b->nq / t.knn_chunk + b->n;
+  int64_t max_items = b->nq / chunk + b->n;
+  unsigned long long* counter = (unsigned long long*)b->knn_counter.ptr;
+  uint32_t *left = nullptr, *left_n = nullptr;
+  if (b->tiles) {
+    // the unsorted keys' place is free
+    left = (uint32_t*)(b->sorted_in_b ? b->qka.ptr : b->qkb.ptr);
+    left_n = (uint32_t*)(counter + 2);
+    const cudaError_t e = batch_tile_launch(
+        b->tables, (const float4*)b->slots.ptr, order, (const int64_t*)b->qoff.ptr,
+        (const int64_t*)b->item_off.ptr, max_items, chunk, b->max_k, (float*)b->res.ptr, left,
+        left_n, b->tile_per_sm, counter + 1, b->num_sms, b->st);
+    if (e != cudaSuccess) return e;
+    max_items = b->nq;
+  }
   return batch_knn_launch(b->tables, (const float4*)b->slots.ptr, order,
                           (const int64_t*)b->qoff.ptr, (const int64_t*)b->item_off.ptr,
                           max_items, (float*)b->res.ptr, t.knn_warps, t.knn_chunk, t.knn_buffer,
-                          per_sm, (unsigned long long*)b->knn_counter.ptr, b->num_sms, b->st);
+                          per_sm, counter, b->num_sms, b->st, left, left_n);
 }
 
 // The whole step with the current tuning (no host synchronisation).
@@ -447,7 +466,7 @@ int plan(pm_batch* b) {
       (s = b->qva.ensure(ts * 4)) || (s = b->qvb.ensure(ts * 4)) ||
       (s = b->qhist.ensure(sort_hist_words((int64_t)ts) * 4)) || (s = b->qcount.ensure(16)) ||
       (s = b->qstart.ensure(8 * (size_t)n)) || (s = b->qoff.ensure(8 * (size_t)(n + 1))) ||
-      (s = b->item_off.ensure(8 * (size_t)(n + 1))) || (s = b->knn_counter.ensure(16)))
+      (s = b->item_off.ensure(8 * (size_t)(n + 1))) || (s = b->knn_counter.ensure(64)))
     return berr(b, s, "camera buffers (%lld query slots)", (long long)b->total_slots);
   if ((s = upload_tables(b)) != PM_OK) return s;
   // 4. queries: the step up to the listing
@@ -461,6 +480,9 @@ int plan(pm_batch* b) {
       (e = cudaStreamSynchronize(b->st)))
     return bcuda(b, e, "batch plan");
   b->nq = nq;
+  b->tiles = b->max_k <= kTileMaxK && b->nq * (b->max_k + 50) >= kTileMinWork / 2;
+  if (b->tiles && (e = batch_tile_prepare(b->max_k, &b->tile_per_sm)))
+    return bcuda(b, e, "kNN set-up");
   if ((e = batch_knn_prepare(b->tune.knn_warps, b->tune.knn_buffer, &b->knn_per_sm)))
     return bcuda(b, e, "kNN set-up");
   // 5. one full step, checked

@@ -26,9 +26,12 @@
 // A query that cannot be answered here (a list that stays too long, more than
 // 16 photons in the k-th bin, fewer than k photons) goes to a list that the
 // warp-per-query kernel answers afterwards.
+#include "pm_batch.cuh"
 #include "pm_knn_tile.cuh"
 
 #include <float.h>
+
+#include <algorithm>
 
 namespace pm {
 
@@ -692,6 +695,60 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
   }
 }
 
+// The same for every scene of a batch: a work item is up to `item` consecutive
+// sorted queries of one scene. A warp switches its copy of the map when the
+// scene changes. Scenes whose map is too small leave their queries. Measured on
+// 8 random scenes (50k to 1M photons emitted, k = 50 and 100): 2.63 ms for the
+// estimates of a step, 7.97 ms by the warp-per-query kernel.
+__global__ void __launch_bounds__(32 * kTileWarps, 5)
+    knn_tile_batch_kernel(BatchTables t, const float4* __restrict__ slots,
+                          const uint32_t* __restrict__ order, const int64_t* __restrict__ qoff,
+                          const int64_t* __restrict__ item_off, int item, float* __restrict__ rgb,
+                          int rows, TileDefer defer, unsigned long long* __restrict__ counter) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int64_t ioff[kMaxBatchScenes + 1];
+  __shared__ MapDev wmap[kTileWarps];
+  __shared__ TileLevels wlev[kTileWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  TileWarp& s = *reinterpret_cast<TileWarp*>(smem_raw + warp * tile_bytes(rows));
+  batch_load_offsets(ioff, item_off, t.n_scenes);
+  __syncthreads();
+  const int64_t total = ioff[t.n_scenes];
+  int cur = -1, k = 0;
+  float tau = 0.f, n_emitted = 0.f;
+  while (true) {
+    unsigned long long c0 = 0;
+    if (lane == 0) c0 = atomicAdd(counter, 1ull);
+    c0 = __shfl_sync(kFull, c0, 0);
+    if ((int64_t)c0 >= total) break;
+    const int sc = batch_find(ioff, t.n_scenes, (int64_t)c0);
+    if (sc != cur) {
+      __syncwarp();
+      const BatchScene& bs = t.scenes[sc];
+      if (lane == 0) wmap[warp] = bs.map;
+      if (lane < kMaxLevels) wlev[warp].oc[lane] = make_int2(bs.map.lvl_off[lane], bs.map.lvl_cnt[lane]);
+      __syncwarp();
+      cur = sc;
+      k = bs.k;
+      n_emitted = bs.n_emitted;
+      if (wmap[warp].n >= kTileMinPhotons)
+        tau = even_tau(wmap[warp], wmap[warp].lvl_off[wmap[warp].nlevels - 1], k);
+    }
+    const int64_t q0 = qoff[sc] + ((int64_t)c0 - ioff[sc]) * item;
+    const int nq = (int)min((int64_t)item, qoff[sc + 1] - q0);
+    if (wmap[warp].n < kTileMinPhotons) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(defer.count, (uint32_t)nq);
+      base = __shfl_sync(kFull, base, 0);
+      if (lane < nq) defer.list[base + lane] = (uint32_t)(q0 + lane);
+      continue;
+    }
+    tile_item(wmap[warp], wlev[warp], s, rows, lane, slots, order, 4, q0, nq, k, n_emitted, rgb,
+              defer, tau);
+    __syncwarp();
+  }
+}
+
 }  // namespace
 
 // Rows of 32 photons that a sub-tile may take: about 8 photons per kept one
@@ -738,6 +795,42 @@ cudaError_t knn_tile_launch(const MapDev& m, const void* queries, int64_t nq, in
     return e;
   knn_tile_kernel<<<(unsigned)blocks, 32 * kTileWarps, smem, st>>>(
       m, (const float4*)queries, order, nq, stride4, k, n_emitted, rgb, rows, item, defer, counter);
+  return cudaGetLastError();
+}
+
+int batch_tile_item(int64_t nq, int num_sms) {
+  int item = kTileQ;
+  while (item > kSubQ && nq < 4 * (int64_t)item * num_sms * 5 * kTileWarps) item >>= 1;
+  return item;
+}
+
+cudaError_t batch_tile_prepare(int max_k, int* blocks_per_sm) {
+  const size_t smem = kTileWarps * tile_bytes(tile_rows(max_k));
+  cudaError_t e = cudaFuncSetAttribute(
+      knn_tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_tile_batch_kernel,
+                                                    32 * kTileWarps, smem);
+  *blocks_per_sm = per_sm < 1 ? 1 : per_sm;
+  return e;
+}
+
+cudaError_t batch_tile_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
+                              const int64_t* qoff, const int64_t* item_off, int64_t max_items,
+                              int item, int max_k, float* res, uint32_t* left, uint32_t* left_n,
+                              int blocks_per_sm, unsigned long long* counter, int num_sms,
+                              cudaStream_t st) {
+  const int rows = tile_rows(max_k);
+  const int64_t need = (max_items + kTileWarps - 1) / kTileWarps;
+  const int64_t blocks =
+      std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)num_sms * blocks_per_sm));
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st)) != cudaSuccess ||
+      (e = cudaMemsetAsync(left_n, 0, sizeof(uint32_t), st)) != cudaSuccess)
+    return e;
+  knn_tile_batch_kernel<<<(unsigned)blocks, 32 * kTileWarps, kTileWarps * tile_bytes(rows), st>>>(
+      t, slots, order, qoff, item_off, item, res, rows, TileDefer{left, left_n, true}, counter);
   return cudaGetLastError();
 }
 

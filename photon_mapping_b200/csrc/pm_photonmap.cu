@@ -1158,16 +1158,17 @@ __global__ void __launch_bounds__(256, 4)
     knn_batch_kernel(BatchTables t, const float4* __restrict__ slots,
                      const uint32_t* __restrict__ order, const int64_t* __restrict__ qoff,
                      const int64_t* __restrict__ item_off, int chunk, KnnOut out,
-                     unsigned long long* __restrict__ counter) {
+                     unsigned long long* __restrict__ counter, const uint32_t* __restrict__ left,
+                     const uint32_t* __restrict__ left_n) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t ioff[kMaxBatchScenes + 1];
   __shared__ MapDev wmap[8];
   __shared__ Levels wlev[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpBuf<C>& s = reinterpret_cast<WarpBuf<C>*>(smem_raw)[warp];
-  batch_load_offsets(ioff, item_off, t.n_scenes);
+  batch_load_offsets(ioff, left ? qoff : item_off, t.n_scenes);
   __syncthreads();
-  const int64_t total = ioff[t.n_scenes];
+  const int64_t total = left ? (int64_t)*left_n : ioff[t.n_scenes];
   float r_hint = -1.f;
   int cur = -1, k = 0;
   float n_emitted = 0.f;
@@ -1176,7 +1177,8 @@ __global__ void __launch_bounds__(256, 4)
     if (lane == 0) c0 = atomicAdd(counter, 1ull);
     c0 = __shfl_sync(kFull, c0, 0);
     if ((int64_t)c0 >= total) break;
-    const int sc = batch_find(ioff, t.n_scenes, (int64_t)c0);
+    const int64_t at = left ? (int64_t)left[c0] : (int64_t)c0;
+    const int sc = batch_find(ioff, t.n_scenes, at);
     if (sc != cur) {
       __syncwarp();
       if (lane == 0) {
@@ -1192,8 +1194,8 @@ __global__ void __launch_bounds__(256, 4)
       n_emitted = t.scenes[sc].n_emitted;
       r_hint = -1.f;
     }
-    const int64_t qb = qoff[sc] + ((int64_t)c0 - ioff[sc]) * chunk;
-    const int64_t qe = min(qoff[sc + 1], qb + chunk);
+    const int64_t qb = left ? at : qoff[sc] + (at - ioff[sc]) * chunk;
+    const int64_t qe = left ? at + 1 : min(qoff[sc + 1], qb + chunk);
     knn_chunk<C, kModeRadiance, false, false>(wmap[warp], wlev[warp], s, lane, slots, qb, qe, k,
                                        n_emitted, out, order, 4, r_hint);
   }
@@ -1216,7 +1218,8 @@ cudaError_t batch_knn_prepare(int warps, int buffer, int* blocks_per_sm) {
 cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
                              const int64_t* qoff, const int64_t* item_off, int64_t max_items,
                              float* res, int warps, int chunk, int buffer, int blocks_per_sm,
-                             unsigned long long* counter, int num_sms, cudaStream_t st) {
+                             unsigned long long* counter, int num_sms, cudaStream_t st,
+                             const uint32_t* left, const uint32_t* left_n) {
   if (warps < 1 || warps > 8 || chunk < 1) return cudaErrorInvalidValue;
   const int threads = 32 * warps;
   auto kern = buffer <= 512 ? knn_batch_kernel<512> : knn_batch_kernel<2048>;
@@ -1231,7 +1234,7 @@ cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const ui
   KnnOut out{};
   out.rgb = res;
   kern<<<(unsigned)blocks, threads, smem, st>>>(t, slots, order, qoff, item_off, chunk, out,
-                                                counter);
+                                                counter, left, left_n);
   return cudaGetLastError();
 }
 
