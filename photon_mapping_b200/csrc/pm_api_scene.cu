@@ -86,7 +86,7 @@ int upload_scene(DevScene& sc, DevBuf& scratch, cudaStream_t st, const float* ve
       (s = sc.geo.ensure(nf * 16)) || (s = sc.mat.ensure(nf * sizeof(Material))) ||
       (s = sc.lights.ensure((lights.size() + 1) * 4)) ||
       (s = sc.mt.ensure(nf * 3 * 16)) ||
-      (s = sc.nodes.ensure((nf > 1 ? nf - 1 : 1) * 4 * 16)) ||
+      (s = sc.nodes.ensure((nf > 1 ? nf - 1 : 1) * 8 * 16)) ||
       (s = scratch.ensure(scene_build_scratch_bytes((int)n))))
     return s;
   cudaError_t e;

@@ -55,7 +55,8 @@ __device__ V3 direct_light(const SceneDev& sc, const Surf& s, V3 wo,
                            const Material& m, Rng& rng) {
   float pc, pp;
   const int lf = sample_light(sc, rng, pc);
-  const Surf ls = sample_triangle(sc, lf, rng, pp);
+  Surf ls;
+  sample_triangle_point(sc, lf, rng, ls.pos, ls.ns, pp);
   const V3 wi = normalize(ls.pos - s.pos);
   const float r = length(ls.pos - s.pos);
   const float pd = pp * r * r / fabsf(dot(-wi, ls.ns));

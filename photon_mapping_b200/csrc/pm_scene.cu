@@ -239,24 +239,77 @@ __global__ void ploc_merge_kernel(const int* __restrict__ cid, const float4* __r
   bhi2[o] = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
 }
 
+// Record i of the tree that walks use (pm_scene.cuh) from the binary nodes
+// {left lo, left child}, {left hi, right child}, {right lo}, {right hi}: the
+// grandchildren of node i, and its children that are leaves.
+__global__ void widen_kernel(const float4* __restrict__ binary, int n, float4* __restrict__ wide) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float4 lo[4], hi[4];
+  int id[4];
+  int m = 0;
+  auto add = [&](const float4& l, const float4& u, int child) {
+    // m is known at compile time in none of the calls: write every slot that
+    // matches
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j == m) {
+        lo[j] = l;
+        hi[j] = u;
+        id[j] = child;
+      }
+    ++m;
+  };
+  const float4* b = binary + 4 * (size_t)i;
+  const float4 b0 = b[0], b1 = b[1], b2 = b[2], b3 = b[3];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int child = __float_as_int(c ? b1.w : b0.w);
+    if (child < 0) {
+      add(c ? b2 : b0, c ? b3 : b1, child);
+    } else {
+      const float4* g = binary + 4 * (size_t)child;
+      const float4 g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3];
+      add(g0, g1, __float_as_int(g0.w));
+      add(g2, g3, __float_as_int(g1.w));
+    }
+  }
+  // absent children: a point far outside (should a ray meet it all the same,
+  // the id says that there is nothing)
+  const float4 far = make_float4(1e38f, -1e38f, 2e38f, 0.f);
+  while (m < 4) add(far, far, kNoChild);
+  float4* w = wide + 8 * (size_t)i;
+  w[0] = make_float4(lo[0].x, lo[1].x, lo[2].x, lo[3].x);
+  w[1] = make_float4(lo[0].y, lo[1].y, lo[2].y, lo[3].y);
+  w[2] = make_float4(lo[0].z, lo[1].z, lo[2].z, lo[3].z);
+  w[3] = make_float4(hi[0].x, hi[1].x, hi[2].x, hi[3].x);
+  w[4] = make_float4(hi[0].y, hi[1].y, hi[2].y, hi[3].y);
+  w[5] = make_float4(hi[0].z, hi[1].z, hi[2].z, hi[3].z);
+  w[6] = make_float4(__int_as_float(id[0]), __int_as_float(id[1]), __int_as_float(id[2]),
+                     __int_as_float(id[3]));
+  w[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 size_t scene_build_scratch_bytes(int n) {
   const size_t nn = (size_t)(n > 1 ? n : 2);
   // cluster boxes a/b (4n float4), sort keys / values a/b (4n), histogram,
   // scene box, cluster ids a/b and neighbours (3n), pass flags and ranks
   // (4n), scan tile sums, pass counts
-  return 4 * nn * 16 + 4 * nn * 4 + sort_hist_words(nn) * 4 + 64 + 3 * nn * 4 + 4 * nn * 4 +
+  // and the binary nodes (4n float4)
+  return 4 * nn * 16 + 4 * nn * 16 + 4 * nn * 4 + sort_hist_words(nn) * 4 + 64 + 3 * nn * 4 + 4 * nn * 4 +
          (size_t)scan_tiles((int64_t)nn) * 4 + 64;
 }
 
 cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, float4* tri,
-                               float4* nrm, float4* geo, float4* mt, float4* nodes,
+                               float4* nrm, float4* geo, float4* mt, float4* wide,
                                void* scratch, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   float4* blo_a = (float4*)scratch;
   float4* bhi_a = blo_a + n;
   float4* blo_b = bhi_a + n;
   float4* bhi_b = blo_b + n;
-  uint32_t* ka = (uint32_t*)(bhi_b + n);
+  float4* nodes = bhi_b + n;
+  uint32_t* ka = (uint32_t*)(nodes + 4 * (size_t)n);
   uint32_t* kb = ka + n;
   uint32_t* va = kb + n;
   uint32_t* vb = va + n;
@@ -308,6 +361,7 @@ cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, flo
     std::swap(bhi_a, bhi_b);
   }
   if (m != 1 || top != 0) return cudaErrorUnknown;
+  widen_kernel<<<(n - 1 + tb - 1) / tb, tb, 0, st>>>(nodes, n - 1, wide);
   return cudaGetLastError();
 }
 

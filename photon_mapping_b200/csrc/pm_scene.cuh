@@ -8,9 +8,12 @@
 //   mat    Material[n] per-face BxDF and emission (scene.h:21-51)
 //   lights int[m]      faces with emission > 0, in face order
 //   mt     float4[3n]  leaf order: {p0, face id}, {p1 - p0}, {p2 - p0}
-//   nodes  float4[4(n-1)] internal nodes: {left box lo, left child},
-//                      {left box hi, right child}, {right box lo},
-//                      {right box hi}; a child < 0 is leaf ~child.
+//   nodes  float4[8(n-1)] one record per inner node i of the binary tree, of its
+//                      up to 4 grandchildren (a child that is a leaf counts
+//                      itself): lo.x, lo.y, lo.z, hi.x, hi.y, hi.z of the four,
+//                      their ids (>= 0: inner node, < 0: leaf ~id, kNoChild:
+//                      none), and 16 bytes of padding to a 128-byte line. A walk
+//                      from node 0 takes two levels of the binary tree per step.
 #pragma once
 
 #include "pm_math.cuh"
@@ -58,21 +61,105 @@ __device__ __forceinline__ bool ray_triangle(V3 o, V3 d, V3 p0, V3 e1, V3 e2,
   return t == t;
 }
 
-// Slab test of the ray against a box; NaN products (0 * inf) impose no
-// constraint. The exit distance is widened by 1 + 2*gamma(3) (Ize 2013)
-// and the boxes themselves are padded at build time, so a box is never
-// culled when a triangle inside it is hit.
-__device__ __forceinline__ bool ray_box(V3 o, V3 inv, float tmin, float tmax,
-                                        float4 lo, float4 hi, float& tnear) {
-  const float tx0 = (lo.x - o.x) * inv.x, tx1 = (hi.x - o.x) * inv.x;
-  const float ty0 = (lo.y - o.y) * inv.y, ty1 = (hi.y - o.y) * inv.y;
-  const float tz0 = (lo.z - o.z) * inv.z, tz1 = (hi.z - o.z) * inv.z;
-  const float tn = fmaxf(fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)),
-                               fminf(tz0, tz1)), tmin);
-  const float tf = fminf(fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)),
-                               fmaxf(tz0, tz1)), tmax);
-  tnear = tn;
-  return tn <= tf * 1.00000072f;
+constexpr int kNoChild = (int)0x80000000;
+
+// Entries of the traversal stack of a walk that the binary tree would give
+// STACK: a step pushes up to 3 where two levels of the binary tree push 2. (16
+// gives 23: a tree of equal boxes that needs 17 of the binary walk is to be
+// refused there, as it always was.)
+template <int STACK>
+__host__ __device__ constexpr int stack_entries() {
+  return STACK + STACK / 2 - (STACK == 16 ? 1 : 0);
+}
+
+// One step of a walk: the boxes of node `node` against the ray (o, inv) in
+// [tmin, tmax]. Returns the inner child entered first (-1: none) and pushes the
+// other inner children hit, the nearest on top; `leaves` gets a bit per leaf
+// child hit, its id in ids.
+//
+// Slab test; NaN products (0 * inf) impose no constraint. The exit distance is
+// widened by 1 + 2*gamma(3) (Ize 2013) and the boxes themselves are padded at
+// build time, so a box is never culled when a triangle inside it is hit. Two
+// boxes at a time in packed arithmetic.
+struct RayPacked {
+  F2 ox, oy, oz, ix, iy, iz;  // minus the origin, and 1 / direction, twice each
+  __device__ __forceinline__ void set(V3 o, V3 d) {
+    ox = f2(-o.x, -o.x), oy = f2(-o.y, -o.y), oz = f2(-o.z, -o.z);
+    const V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    ix = f2(inv.x, inv.x), iy = f2(inv.y, inv.y), iz = f2(inv.z, inv.z);
+  }
+};
+
+// Largest / smallest of three (NaN ignored), one instruction.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+template <int N>
+__device__ __forceinline__ int walk_step(const float4* __restrict__ nodes, int node,
+                                         const RayPacked& r, float tmin, float tmax,
+                                         int (&stack)[N], int& sp, int* err, unsigned& leaves,
+                                         int4& ids) {
+  const ulonglong2* n = reinterpret_cast<const ulonglong2*>(nodes + 8 * (size_t)node);
+  const ulonglong2 lx = __ldg(n), ly = __ldg(n + 1), lz = __ldg(n + 2);
+  const ulonglong2 hx = __ldg(n + 3), hy = __ldg(n + 4), hz = __ldg(n + 5);
+  ids = __ldg(reinterpret_cast<const int4*>(n + 6));
+  uint32_t key[4];  // entry distance of inner children hit, index in the low bits
+  leaves = 0;
+  const int id[4] = {ids.x, ids.y, ids.z, ids.w};
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const float2 x0 = f2_split(f2_mul(f2_add(p ? lx.y : lx.x, r.ox), r.ix));
+    const float2 x1 = f2_split(f2_mul(f2_add(p ? hx.y : hx.x, r.ox), r.ix));
+    const float2 y0 = f2_split(f2_mul(f2_add(p ? ly.y : ly.x, r.oy), r.iy));
+    const float2 y1 = f2_split(f2_mul(f2_add(p ? hy.y : hy.x, r.oy), r.iy));
+    const float2 z0 = f2_split(f2_mul(f2_add(p ? lz.y : lz.x, r.oz), r.iz));
+    const float2 z1 = f2_split(f2_mul(f2_add(p ? hz.y : hz.x, r.oz), r.iz));
+    const float na = fmaxf(max3(fminf(x0.x, x1.x), fminf(y0.x, y1.x), fminf(z0.x, z1.x)), tmin);
+    const float nb = fmaxf(max3(fminf(x0.y, x1.y), fminf(y0.y, y1.y), fminf(z0.y, z1.y)), tmin);
+    const float fa = fminf(min3(fmaxf(x0.x, x1.x), fmaxf(y0.x, y1.x), fmaxf(z0.x, z1.x)), tmax);
+    const float fb = fminf(min3(fmaxf(x0.y, x1.y), fmaxf(y0.y, y1.y), fmaxf(z0.y, z1.y)), tmax);
+    const bool ha = na <= fa * 1.00000072f, hb = nb <= fb * 1.00000072f;
+    const int i = 2 * p;
+    key[i] = ha && id[i] >= 0 ? (__float_as_uint(na) & ~3u) | (unsigned)i : 0xffffffffu;
+    key[i + 1] = hb && id[i + 1] >= 0 ? (__float_as_uint(nb) & ~3u) | (unsigned)(i + 1) : 0xffffffffu;
+    if (ha && id[i] < 0) leaves |= 1u << i;
+    if (hb && id[i + 1] < 0) leaves |= 2u << i;
+  }
+  // nearest first (a network of 5 exchanges)
+  auto order = [](uint32_t& a, uint32_t& b) {
+    const uint32_t l = min(a, b);
+    b = max(a, b);
+    a = l;
+  };
+  order(key[0], key[1]);
+  order(key[2], key[3]);
+  order(key[0], key[2]);
+  order(key[1], key[3]);
+  order(key[1], key[2]);
+  auto child = [&](uint32_t k) {
+    const int lo = k & 1u ? ids.y : ids.x, hi = k & 1u ? ids.w : ids.z;
+    return k & 2u ? hi : lo;
+  };
+  // the others, the farthest first
+  const int more = (key[1] != 0xffffffffu) + (key[2] != 0xffffffffu) + (key[3] != 0xffffffffu);
+  if (sp + more <= N) {
+    if (more > 0) stack[sp + more - 1] = child(key[1]);
+    if (more > 1) stack[sp + more - 2] = child(key[2]);
+    if (more > 2) stack[sp] = child(key[3]);
+    sp += more;
+  } else {
+    atomicOr(err, 1);  // their subtrees are lost
+  }
+  if (key[0] != 0xffffffffu) return child(key[0]);
+  return sp > 0 ? stack[--sp] : -1;
 }
 
 __device__ __forceinline__ void test_leaf(const SceneDev& sc, int leaf, V3 o,
@@ -107,49 +194,21 @@ __device__ __forceinline__ bool intersect_t(const SceneDev& sc, V3 o, V3 d,
     test_leaf(sc, 0, o, d, tmin, h);
     return h.prim >= 0;
   }
-  const V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-  int stack[STACK];
+  RayPacked r;
+  r.set(o, d);
+  int stack[stack_entries<STACK>()];
   int sp = 0;
   int node = 0;
-  while (true) {
-    const float4 a = __ldg(sc.nodes + 4 * node);
-    const float4 b = __ldg(sc.nodes + 4 * node + 1);
-    const float4 c = __ldg(sc.nodes + 4 * node + 2);
-    const float4 e = __ldg(sc.nodes + 4 * node + 3);
-    const int left = __float_as_int(a.w), right = __float_as_int(b.w);
-    float tl, tr;
-    const bool hl = ray_box(o, inv, tmin, h.t, a, b, tl);
-    const bool hr = ray_box(o, inv, tmin, h.t, c, e, tr);
-    int next = -1, other = -1;
-    if (hl) {
-      if (left < 0) test_leaf(sc, ~left, o, d, tmin, h);
-      else next = left;
-    }
-    if (hr) {
-      if (right < 0) {
-        test_leaf(sc, ~right, o, d, tmin, h);
-      } else if (next < 0) {
-        next = right;
-      } else {
-        other = right;
-        if (tr < tl) {
-          other = next;
-          next = right;
-        }
-      }
-    }
-    if (other >= 0) {
-      if (sp < STACK) {
-        stack[sp++] = other;
-      } else {
-        atomicOr(sc.err, 1);
-      }
-    }
-    if (next < 0) {
-      if (sp == 0) break;
-      node = stack[--sp];
-    } else {
-      node = next;
+  while (node >= 0) {
+    unsigned leaves;
+    int4 ids;
+    node = walk_step(sc.nodes, node, r, tmin, h.t, stack, sp, sc.err, leaves, ids);
+    while (leaves) {
+      const int i = __ffs(leaves) - 1;
+      leaves &= leaves - 1;
+      const int lo = i & 1 ? ids.y : ids.x, hi = i & 1 ? ids.w : ids.z;
+      const int id = i & 2 ? hi : lo;
+      if (id != kNoChild) test_leaf(sc, ~id, o, d, tmin, h);
     }
   }
   return h.prim >= 0;
@@ -159,6 +218,68 @@ __device__ __forceinline__ bool intersect(const SceneDev& sc, V3 o, V3 d,
                                           float tmin, float tmax, Hit& h) {
   return intersect_t<kBvhStack>(sc, o, d, tmin, tmax, h);
 }
+
+// A closest-hit query in progress, for kernels that let the lanes of a warp
+// work on rays of different lengths (pm_trace.cu). The result is that of
+// intersect_t: the same boxes and triangles are tested with the same arithmetic,
+// in an order that does not matter. The stack (kept beside it: an array indexed
+// at run time would take the whole struct out of registers) holds the same
+// entries.
+struct Walk {
+  const float4* nodes;
+  const float4* mt;
+  RayPacked r;
+  float tmin;
+  Hit h;
+  int node;         // inner node to visit next, -1: none
+  unsigned leaves;  // leaf children of the last node that are still to be tested
+  int4 ids;         // the ids of that node's children
+  int sp;
+
+  __device__ __forceinline__ bool at_leaf() const { return leaves != 0u; }
+  __device__ __forceinline__ bool over() const { return node < 0 && leaves == 0u; }
+
+  __device__ __forceinline__ void start(const SceneDev& sc, V3 ro, V3 rd, float t0, float t1) {
+    nodes = sc.nodes;
+    mt = sc.mt;
+    r.set(ro, rd);
+    tmin = t0;
+    h.t = t1;
+    h.prim = -1;
+    h.u = h.v = 0.f;
+    sp = 0;
+    node = sc.n_faces > 1 ? 0 : -1;
+    leaves = sc.n_faces == 1 ? 1u : 0u;
+    ids = make_int4(~0, 0, 0, 0);
+  }
+
+  // Visits `node` (>= 0, no leaf waiting).
+  template <int N>
+  __device__ __forceinline__ void visit(int (&stack)[N], int* err) {
+    node = walk_step(nodes, node, r, tmin, h.t, stack, sp, err, leaves, ids);
+  }
+
+  // Tests the first leaf that waits against the ray (o, d) given to start().
+  __device__ __forceinline__ void test(V3 o, V3 d) {
+    const int i = __ffs(leaves) - 1;
+    leaves &= leaves - 1;
+    const int lo = i & 1 ? ids.y : ids.x, hi = i & 1 ? ids.w : ids.z;
+    const int id = i & 2 ? hi : lo;
+    if (id == kNoChild) return;
+    const float4* leaf = mt + 3 * (size_t)~id;
+    const float4 a = __ldg(leaf), b = __ldg(leaf + 1), c = __ldg(leaf + 2);
+    float t, u, v;
+    if (ray_triangle(o, d, f4v3(a), f4v3(b), f4v3(c), t, u, v)) {
+      const int prim = __float_as_int(a.w);
+      if (t >= tmin && t <= h.t && (t < h.t || h.prim < 0 || prim < h.prim)) {
+        h.t = t;
+        h.u = u;
+        h.v = v;
+        h.prim = prim;
+      }
+    }
+  }
+};
 
 // Surface frame at a hit (scene.h:324-337): position = ray(t), shading
 // normal interpolated and not re-normalised (triangle.h:64-71), tangent
@@ -187,8 +308,8 @@ __device__ __forceinline__ Surf surface_at(const SceneDev& sc, V3 o, V3 d,
 
 // Triangle::samplePoint (triangle.h:84-114): uniform point, pdf = 1/area.
 // Draws one getNext2D.
-__device__ __forceinline__ Surf sample_triangle(const SceneDev& sc, int f,
-                                                Rng& rng, float& pdf) {
+__device__ __forceinline__ void sample_triangle_point(const SceneDev& sc, int f, Rng& rng, V3& pos,
+                                                      V3& ns, float& pdf) {
   float u0, u1;
   rng.next2d(u0, u1);
   const float su0 = sqrtf(u0);
@@ -196,13 +317,9 @@ __device__ __forceinline__ Surf sample_triangle(const SceneDev& sc, int f,
   const V3 p1 = f4v3(__ldg(sc.tri + 3 * f));
   const V3 p2 = f4v3(__ldg(sc.tri + 3 * f + 1));
   const V3 p3 = f4v3(__ldg(sc.tri + 3 * f + 2));
-  Surf s;
-  s.pos = (1.0f - b0 - b1) * p1 + b0 * p2 + b1 * p3;
-  s.ns = shading_normal(sc, f, b0, b1);
-  orthonormal_basis(s.ns, s.dpdu, s.dpdv);
-  s.ng = f4v3(__ldg(sc.geo + f));
+  pos = (1.0f - b0 - b1) * p1 + b0 * p2 + b1 * p3;
+  ns = shading_normal(sc, f, b0, b1);
   pdf = 1.0f / __ldg(sc.geo + f).w;
-  return s;
 }
 
 // Scene::sampleLight (scene.h:350-355): uniform over the light faces by

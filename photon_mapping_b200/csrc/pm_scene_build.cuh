@@ -9,7 +9,7 @@ namespace pm {
 size_t scene_build_scratch_bytes(int n);
 
 // verts / nrms: device, 9 floats per face. Fills tri, nrm, geo (face
-// order), mt (leaf order) and nodes (n - 1 internal nodes). Synchronises st
+// order), mt (leaf order) and nodes (n - 1 records of 8 float4). Synchronises st
 // once per clustering pass (it reads the clusters left).
 cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, float4* tri,
                                float4* nrm, float4* geo, float4* mt, float4* nodes,

@@ -67,57 +67,42 @@ struct PhotonPath {
   bool prev_specular;
 };
 
-// sampleRayFromLight (integrator.h:265-288): the start of photon i.
-template <int MODE>
+// A point at which a path's next direction is drawn: on a light (the start of
+// a photon) or on the surface a ray has hit.
+struct PathVertex {
+  V3 pos, ns, ng;
+  int face;
+  float pdf_point;  // light: of the face times of the point on it
+};
+
+// The first half of sampleRayFromLight (integrator.h:265-288): the starting
+// point of photon i.
 __device__ __forceinline__ void photon_emit(const SceneDev& sc, const TraceArgs& a, int i,
-                                            PhotonPath& p) {
+                                            PhotonPath& p, PathVertex& v) {
   p.rng = Rng{photon_stream_state(a.seed, (unsigned long long)i)};
-  float pdf_choose, pdf_pos, pdf_dir;
-  const int lf = sample_light(sc, p.rng, pdf_choose);
-  const Surf ls = sample_triangle(sc, lf, p.rng, pdf_pos);
-  float u0, u1;
-  p.rng.next2d(u0, u1);
-  const V3 dl = sample_cos_hemisphere(u0, u1, pdf_dir);
-  p.dir = local_to_world(dl, ls.dpdu, ls.ns, ls.dpdv);
-  const Material& lm = sc.mat[lf];
-  p.thr = v3(lm.le[0], lm.le[1], lm.le[2]) /
-          (pdf_choose * pdf_pos * pdf_dir) * fabsf(dot(p.dir, ls.ns));
-  // decision throughput: the same arithmetic over the decision materials
-  p.td = p.thr;
-  if (MODE != kTracePlain) {
-    const Material& dm = a.dmat[lf];
-    p.td = v3(dm.le[0], dm.le[1], dm.le[2]) /
-           (pdf_choose * pdf_pos * pdf_dir) * fabsf(dot(p.dir, ls.ns));
-  }
-  p.org = ls.pos;
+  float pdf_choose, pdf_pos;
+  v.face = sample_light(sc, p.rng, pdf_choose);
+  sample_triangle_point(sc, v.face, p.rng, v.pos, v.ns, pdf_pos);
+  v.pdf_point = pdf_choose * pdf_pos;
   p.i = i;
   p.k = 0;
   p.nst = 0;
   p.prev_specular = false;
 }
 
-// One iteration k of the tracing loop (integrator.h:417-468 global,
-// :497-557 caustics); false when the path ends.
-template <int MODE, int STACK>
-__device__ __forceinline__ bool photon_step(const SceneDev& sc, const TraceArgs& a,
-                                            PhotonPath& p, ReplaySmem* rs, unsigned& nrays) {
-  if (p.k >= a.max_depth) return false;
+// What an iteration of the tracing loop (integrator.h:417-468 global, :497-557
+// caustics) does with its ray's closest hit h before it draws a direction; false
+// when the path ends.
+template <int MODE>
+__device__ __forceinline__ bool photon_hit(const SceneDev& sc, const TraceArgs& a, PhotonPath& p,
+                                           const Hit& h, ReplaySmem* rs, PathVertex& v) {
+  if (h.prim < 0) return false;  // photon goes to the sky
   const V3 dec = MODE != kTracePlain ? p.td : p.thr;
-  if (has_nan(dec)) {
-    if (MODE != kTraceReplay) atomicAdd(a.status + 0, 1u);
-    return false;
-  }
-  if (dec.x < 0.f || dec.y < 0.f || dec.z < 0.f) {
-    if (MODE != kTraceReplay) atomicAdd(a.status + 1, 1u);
-    return false;
-  }
-  Hit h;
-  ++nrays;
-  if (!intersect_t<STACK>(sc, p.org, p.dir, kRayEps, __int_as_float(0x7f7fffff), h))
-    return false;  // photon goes to the sky
-  const Surf s = surface_at(sc, p.org, p.dir, h);
-  const Material& m = sc.mat[h.prim];
-  const bool diffuse = m.type == kLambert;
+  v.face = h.prim;
+  v.pos = p.org + h.t * p.dir;  // surface_at
+  v.ng = f4v3(__ldg(sc.geo + h.prim));
+  v.ns = shading_normal(sc, h.prim, h.u, h.v);
+  const bool diffuse = sc.mat[h.prim].type == kLambert;
   bool store = false, stop = false;
   if (!a.caustic) {
     store = diffuse;
@@ -146,7 +131,7 @@ __device__ __forceinline__ bool photon_step(const SceneDev& sc, const TraceArgs&
         }
       }
     } else {
-      store_photon(a, p.i, p.nst, p.thr, s.pos, -p.dir);
+      store_photon(a, p.i, p.nst, p.thr, v.pos, -p.dir);
     }
     ++p.nst;
   }
@@ -158,76 +143,165 @@ __device__ __forceinline__ bool photon_step(const SceneDev& sc, const TraceArgs&
     p.thr = p.thr / q;
     if (MODE != kTracePlain) p.td = p.td / q;
   }
-  // Primitive::sampleBxDF FROM_LIGHT (primitive.h:46-62)
-  const V3 wo = -p.dir;
-  const V3 wo_l = world_to_local(wo, s.dpdu, s.ns, s.dpdv);
-  V3 wi_l;
-  float pdf;
-  const V3 f = bxdf_sample(m, wo_l, kFromLight, p.rng, wi_l, pdf);
-  const V3 wi = local_to_world(wi_l, s.dpdu, s.ns, s.dpdv);
-  const float ct = cos_term(wo, wi, s.ns, s.ng, kFromLight);
-  p.thr = p.thr * (f * ct / pdf);
-  if (MODE != kTracePlain) {
-    // albedo parameters sit on Lambert faces only; the direction drawn
-    // does not depend on the albedo
-    const V3 fd = diffuse ? lambert_eval(a.dmat[h.prim], wo_l, wi_l) : f;
-    p.td = p.td * (fd * ct / pdf);
-  }
-  if (MODE == kTraceReplay) {
-    const int pid = a.face_pid[h.prim];
-    if (pid >= 0) ++rs->cnt[pid][threadIdx.x];
-  }
-  p.org = s.pos;
-  p.dir = wi;
-  ++p.k;
   return true;
 }
 
-// Persistent tracing with regeneration: paths end after very different
-// numbers of bounces (Russian roulette, escapes), so instead of one photon
-// per thread, a thread whose path ended takes the next photon index (one
-// atomic per warp for all its lanes that need one) and the warp keeps its
-// lanes busy until the indices run out. The photons traced, and what they
-// store, do not depend on which thread traces them.
+// Draws the direction at vertex v and updates the path: the second half of
+// sampleRayFromLight at a light, Primitive::sampleBxDF FROM_LIGHT
+// (primitive.h:46-62) on a surface. Lights and Lambert surfaces draw the same
+// way, so starting and bouncing lanes run this together.
+template <int MODE>
+__device__ __forceinline__ void photon_leave(const SceneDev& sc, const TraceArgs& a, PhotonPath& p,
+                                             const PathVertex& v, bool light, ReplaySmem* rs) {
+  V3 dpdu, dpdv;
+  orthonormal_basis(v.ns, dpdu, dpdv);
+  const Material& m = sc.mat[v.face];
+  const bool cosine = light || m.type == kLambert;
+  V3 l = v3(0.f, 0.f, 0.f);  // sampled direction in the frame of ns
+  float pdf = 1.f;
+  if (cosine) {
+    float u0, u1;
+    p.rng.next2d(u0, u1);
+    l = sample_cos_hemisphere(u0, u1, pdf);
+  }
+  if (light) {
+    p.dir = local_to_world(l, dpdu, v.ns, dpdv);
+    const float pr = v.pdf_point * pdf;
+    const float c = fabsf(dot(p.dir, v.ns));
+    p.thr = v3(m.le[0], m.le[1], m.le[2]) / pr * c;
+    // decision throughput: the same arithmetic over the decision materials
+    p.td = p.thr;
+    if (MODE != kTracePlain) {
+      const Material& dm = a.dmat[v.face];
+      p.td = v3(dm.le[0], dm.le[1], dm.le[2]) / pr * c;
+    }
+  } else {
+    const V3 wo = -p.dir;
+    const V3 wo_l = world_to_local(wo, dpdu, v.ns, dpdv);
+    V3 f;
+    if (cosine) f = lambert_eval(m, wo_l, l);
+    else f = bxdf_sample(m, wo_l, kFromLight, p.rng, l, pdf);
+    const V3 wi = local_to_world(l, dpdu, v.ns, dpdv);
+    const float ct = cos_term(wo, wi, v.ns, v.ng, kFromLight);
+    p.thr = p.thr * (f * ct / pdf);
+    if (MODE != kTracePlain) {
+      // albedo parameters sit on Lambert faces only; the direction drawn
+      // does not depend on the albedo
+      const V3 fd = cosine ? lambert_eval(a.dmat[v.face], wo_l, l) : f;
+      p.td = p.td * (fd * ct / pdf);
+    }
+    if (MODE == kTraceReplay) {
+      const int pid = a.face_pid[v.face];
+      if (pid >= 0) ++rs->cnt[pid][threadIdx.x];
+    }
+    p.dir = wi;
+    ++p.k;
+  }
+  p.org = v.pos;
+}
+
+// Whether iteration k of the tracing loop traces a ray; false when the path ends
+// there.
+template <int MODE>
+__device__ __forceinline__ bool photon_ray(const TraceArgs& a, const PhotonPath& p) {
+  if (p.k >= a.max_depth) return false;
+  const V3 dec = MODE != kTracePlain ? p.td : p.thr;
+  if (has_nan(dec)) {
+    if (MODE != kTraceReplay) atomicAdd(a.status + 0, 1u);
+    return false;
+  }
+  if (dec.x < 0.f || dec.y < 0.f || dec.z < 0.f) {
+    if (MODE != kTraceReplay) atomicAdd(a.status + 1, 1u);
+    return false;
+  }
+  return true;
+}
+
+// Persistent tracing in which every lane runs at its own pace. Paths end after
+// very different numbers of bounces and rays after very different numbers of
+// nodes, so a lane that has finished its ray does not wait for the others':
+//   * a lane whose path ended takes the next photon index (one atomic per warp
+//     for all its lanes that need one);
+//   * lanes with a ray visit nodes until `shade` lanes have their closest hit;
+//     those shade and start their next ray while the others keep their place in
+//     the tree;
+//   * leaves met are tested together, once `test` lanes wait for one.
+// The photons traced, and what they store, do not depend on which thread traces
+// them or in which order.
 // scene(src) and args(src) give the scene and trace arguments of source src
 // (a scene of a batch, or the kernel's only one); first(g, src) maps the
 // work index g to (source, photon index).
 template <int MODE, int STACK, class Scene, class Args, class First>
 __device__ __forceinline__ void trace_persistent(unsigned long long* next, long long total,
-                                                 ReplaySmem* rs, Scene&& scene, Args&& args,
-                                                 First&& first) {
+                                                 int shade, int test, ReplaySmem* rs,
+                                                 Scene&& scene, Args&& args, First&& first) {
   const int lane = (int)(threadIdx.x & 31);
   PhotonPath p;
+  Walk w;
+  int stack[stack_entries<STACK>()];
   int src = 0;
   long long g = 0;  // work index of the current path
-  bool live = false, done = false;
+  // a lane needs a path, walks the tree with a ray, has its hit, or is done
+  enum { kNeed, kWalk, kHit, kDone };
+  int state = kNeed;
   unsigned nrays = 0;  // closest-hit queries of this thread
   while (true) {
-    const unsigned want = __ballot_sync(kFull, !live && !done);
+    PathVertex v;
+    bool leave = false;  // the lane has a vertex to go on from
+    if (state == kHit) {
+      const TraceArgs& a = args(src);
+      leave = photon_hit<MODE>(scene(src), a, p, w.h, rs, v);
+      if (!leave) {
+        if (MODE != kTraceReplay && a.store_count) a.store_count[g] = (uint32_t)p.nst;
+        state = kNeed;
+      }
+    }
+    const unsigned want = __ballot_sync(kFull, state == kNeed);
+    bool light = false;
     if (want) {
       unsigned long long base = 0;
       const int leader = __ffs(want) - 1;
       if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(want));
       base = __shfl_sync(kFull, base, leader);
-      if (!live && !done) {
+      if (state == kNeed) {
         g = (long long)(base + (unsigned)__popc(want & lt_mask(lane)));
         if (g < total) {
           const int i = first(g, src);
-          photon_emit<MODE>(scene(src), args(src), i, p);
+          photon_emit(scene(src), args(src), i, p, v);
           if (MODE == kTraceReplay)
             for (int j = 0; j < args(src).n_params; ++j) rs->cnt[j][threadIdx.x] = 0;
-          live = true;
+          light = leave = true;
         } else {
-          done = true;
+          state = kDone;
         }
       }
     }
-    if (__ballot_sync(kFull, live) == 0) break;
-    if (live) {
-      live = photon_step<MODE, STACK>(scene(src), args(src), p, rs, nrays);
-      if (!live && MODE != kTraceReplay) {
-        uint32_t* sc = args(src).store_count;
-        if (sc) sc[g] = (uint32_t)p.nst;
+    if (leave) {
+      const SceneDev& sc = scene(src);
+      const TraceArgs& a = args(src);
+      photon_leave<MODE>(sc, a, p, v, light, rs);
+      if (photon_ray<MODE>(a, p)) {
+        w.start(sc, p.org, p.dir, kRayEps, __int_as_float(0x7f7fffff));
+        ++nrays;
+        state = kWalk;
+      } else {
+        if (MODE != kTraceReplay && a.store_count) a.store_count[g] = (uint32_t)p.nst;
+        state = kNeed;
+      }
+    }
+    const int live = __popc(__ballot_sync(kFull, state != kDone));
+    if (live == 0) break;
+    // lanes with a hit that end the walk (fewer when lanes are done)
+    const int enough = max(1, shade * live / 32);
+    while (true) {
+      if (state == kWalk && w.over()) state = kHit;
+      const unsigned walking = __ballot_sync(kFull, state == kWalk);
+      if (walking == 0 || live - __popc(walking) >= enough) break;
+      const unsigned leaf = __ballot_sync(kFull, state == kWalk && w.at_leaf());
+      if (__popc(leaf) >= test || leaf == walking) {
+        if (state == kWalk && w.at_leaf()) w.test(p.org, p.dir);
+      } else {
+        if (state == kWalk && !w.at_leaf()) w.visit(stack, scene(src).err);
       }
     }
   }
@@ -239,8 +313,8 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(128)
-    trace_kernel(SceneDev sc, TraceArgs a) {
+__global__ void __launch_bounds__(128, 6)
+    trace_kernel(SceneDev sc, TraceArgs a, int shade, int test) {
   auto scene = [&](int) -> const SceneDev& { return sc; };
   auto args = [&](int) -> const TraceArgs& { return a; };
   auto first = [](long long g, int& src) {
@@ -251,21 +325,21 @@ __global__ void __launch_bounds__(128)
     __shared__ ReplaySmem rs;
     for (int t = threadIdx.x; t < 3 * a.n_params; t += blockDim.x) rs.g[t] = 0.f;
     __syncthreads();
-    trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, &rs, scene, args, first);
+    trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, shade, test, &rs, scene, args, first);
     __syncthreads();
     for (int t = threadIdx.x; t < 3 * a.n_params; t += blockDim.x)
       if (rs.g[t] != 0.f) atomicAdd(a.grad + t, (double)rs.g[t]);
     return;
   }
-  trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, nullptr, scene, args, first);
+  trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, shade, test, nullptr, scene, args, first);
 }
 
 // Every emitted photon of every scene of a batch: the global map rule, each
 // scene appending to its own region. Persistent: the photon index runs over
 // all scenes' photons, the scene found by binary search.
 template <int STACK>
-__global__ void __launch_bounds__(256)
-    batch_trace_kernel(BatchTables t, int64_t total) {
+__global__ void __launch_bounds__(256, 3)
+    batch_trace_kernel(BatchTables t, int64_t total, int shade, int test) {
   __shared__ int64_t off[kMaxBatchScenes + 1];
   batch_load_offsets(off, t.emit_off, t.n_scenes);
   __syncthreads();
@@ -275,7 +349,7 @@ __global__ void __launch_bounds__(256)
     src = batch_find(off, t.n_scenes, g);
     return (int)(g - off[src]);
   };
-  trace_persistent<kTracePlain, STACK>(t.next_photon, total, nullptr, scene, args, first);
+  trace_persistent<kTracePlain, STACK>(t.next_photon, total, shade, test, nullptr, scene, args, first);
 }
 
 static int sm_count() {
@@ -285,6 +359,18 @@ static int sm_count() {
   return sms;
 }
 
+// Lanes with a hit that end a walk, and lanes at a leaf that start a test
+// (trace_persistent). With several paths per resident lane (24 warps per SM)
+// warps stay full and 20 of 32 is the best (1M photons: caustics scene 4.76 ->
+// 3.56 ms, Cornell box 1.04 -> 0.97 ms; 16 and 24 within 6 %); with fewer, the
+// time is that of the longest paths, which waiting lanes would stretch (100k
+// photons in the box: 0.27 ms, 0.31 ms with 20).
+static void trace_pace(int64_t paths, int* shade, int* test) {
+  const bool full = paths >= 4 * (int64_t)sm_count() * 24 * 32;
+  *shade = full ? 20 : 32;
+  *test = full ? 8 : 1;
+}
+
 void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int stack,
                         cudaStream_t st) {
   if (total_emit <= 0) return;
@@ -292,12 +378,14 @@ void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int
   const long long cap = (long long)sm_count() * (2048 / block);
   const unsigned gb = (unsigned)std::min<long long>(cap, (total_emit + block - 1) / block);
   cudaMemsetAsync(t.next_photon, 0, sizeof(unsigned long long), st);
+  int shade, test;
+  trace_pace(total_emit, &shade, &test);
   if (stack <= 16)
-    batch_trace_kernel<16><<<gb, block, 0, st>>>(t, total_emit);
+    batch_trace_kernel<16><<<gb, block, 0, st>>>(t, total_emit, shade, test);
   else if (stack <= 32)
-    batch_trace_kernel<32><<<gb, block, 0, st>>>(t, total_emit);
+    batch_trace_kernel<32><<<gb, block, 0, st>>>(t, total_emit, shade, test);
   else
-    batch_trace_kernel<64><<<gb, block, 0, st>>>(t, total_emit);
+    batch_trace_kernel<64><<<gb, block, 0, st>>>(t, total_emit, shade, test);
 }
 
 void trace_launch(const SceneDev& sc, const TraceArgs& a, cudaStream_t st) {
@@ -307,12 +395,14 @@ void trace_launch(const SceneDev& sc, const TraceArgs& a, cudaStream_t st) {
   const long long cap = (long long)sm_count() * (2048 / tb);
   const int gb = (int)std::min<long long>(cap, (a.n_emit + tb - 1) / tb);
   cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), st);
+  int shade, test;
+  trace_pace(a.n_emit, &shade, &test);
   if (a.adj)
-    trace_kernel<kTraceReplay><<<gb, tb, 0, st>>>(sc, a);
+    trace_kernel<kTraceReplay><<<gb, tb, 0, st>>>(sc, a, shade, test);
   else if (a.dmat)
-    trace_kernel<kTraceFrozen><<<gb, tb, 0, st>>>(sc, a);
+    trace_kernel<kTraceFrozen><<<gb, tb, 0, st>>>(sc, a, shade, test);
   else
-    trace_kernel<kTracePlain><<<gb, tb, 0, st>>>(sc, a);
+    trace_kernel<kTracePlain><<<gb, tb, 0, st>>>(sc, a, shade, test);
 }
 
 // out[first[p] + j] = the record with key p << 8 | j.
