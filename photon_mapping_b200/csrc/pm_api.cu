@@ -243,6 +243,7 @@ int pm_ctx_destroy(pm_ctx* c) {
     cudaStreamSynchronize(c->stream);
     c->release_all();
     cudaStreamDestroy(c->stream);
+    if (c->side) cudaStreamDestroy(c->side);
   }
   delete c;
   return PM_OK;

@@ -30,7 +30,7 @@ static_assert(PM_BATCH_MAX_SCENES == kMaxBatchScenes, "batch limit");
 struct pm_batch {
   std::mutex mu;  // calls on one batch are serialised
   int device = 0, num_sms = 148;
-  cudaStream_t st = nullptr;
+  cudaStream_t st = nullptr, side = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string err;
   int n = 0;
@@ -77,6 +77,7 @@ struct pm_batch {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (st) cudaStreamDestroy(st);
+    if (side) cudaStreamDestroy(side);
   }
 };
 
@@ -549,8 +550,9 @@ int pm_batch_create(int device, const pm_batch_scene* scenes, int32_t n, pm_batc
   for (int i = 0; i < n; ++i) {
     const pm_batch_scene& d = scenes[i];
     const char* what = "";
-    if ((s = upload_scene(b->scenes[i], b->scene_scratch, b->st, d.vertices, d.normals,
-                          d.materials, d.n_faces, &what)) != PM_OK)
+    if ((s = upload_scene(b->scenes[i], b->scene_scratch, b->st, b->side, d.vertices, d.normals,
+                          d.materials, scan_materials(d.materials, d.n_faces), d.n_faces,
+                          &what)) != PM_OK)
       return berr(b, s, "scene %d: %s", i, what);
     if (d.n_photons > 0 && b->scenes[i].n_lights == 0)
       return berr(b, PM_ERR_INVALID_ARGUMENT, "scene %d has no area light", i);

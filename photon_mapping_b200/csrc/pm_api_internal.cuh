@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/pm_cuda.h"
 #include "pm_photonmap.cuh"
@@ -130,6 +131,7 @@ struct pm_ctx {
   int device = 0;
   int num_sms = 148;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // scene uploads beside the tree build
   std::mutex mu;
   std::string err;
   pm::DevMap maps[2];
@@ -190,11 +192,21 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
 // are sorted in either case).
 bool use_tiles(const pm_ctx* c, const DevMap& dm, int64_t nq, int k, bool sorted);
 int take_device_error(pm_ctx* c, const char* where);
-// Uploads a scene and builds its BVH on stream st (synchronises st). On
-// failure returns the status and names the step in *what.
-int upload_scene(DevScene& sc, DevBuf& scratch, cudaStream_t st, const float* vertices,
-                 const float* normals, const pm_material* materials, int64_t n,
-                 const char** what);
+// What one pass over the face materials finds (bad: the first face with an
+// unknown type, -1 for none).
+struct SceneFaces {
+  std::vector<int> lights;
+  bool has_specular = false;
+  int64_t bad = -1;
+};
+SceneFaces scan_materials(const pm_material* materials, int64_t n);
+// Uploads a scene and builds its BVH on stream st, with uploads on stream side
+// (created when null) next to it; synchronises both. On failure returns the
+// status and names the step in *what.
+int upload_scene(DevScene& sc, DevBuf& scratch, cudaStream_t st, cudaStream_t& side,
+                 const float* vertices,
+                 const float* normals, const pm_material* materials, const SceneFaces& faces,
+                 int64_t n, const char** what);
 // Traces `map` (the body of pm_photons_trace; the caller holds the lock).
 // dmat: decision materials (frozen decisions) or null; first: receives the
 // first stored photon of each emitted photon, or null.

@@ -6,34 +6,42 @@
 #include "pm_scene_build.cuh"
 #include "pm_sort.cuh"
 
+#include <cooperative_groups.h>
 #include <float.h>
 
-#include <utility>
+#include <algorithm>
+#include <cstring>
 
 namespace pm {
 
 // Per-face constants (triangle.h:25-34) and the leaf records.
-__global__ void face_setup_kernel(const float* __restrict__ verts,
-                                  const float* __restrict__ nrms, int n,
+__global__ void face_setup_kernel(const float* __restrict__ verts, int n,
                                   float4* __restrict__ tri,
-                                  float4* __restrict__ nrm,
                                   float4* __restrict__ geo) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= n) return;
   const float* v = verts + 9 * (size_t)f;
-  const float* nn = nrms + 9 * (size_t)f;
   const V3 p1 = v3(v[0], v[1], v[2]);
   const V3 p2 = v3(v[3], v[4], v[5]);
   const V3 p3 = v3(v[6], v[7], v[8]);
   tri[3 * f] = make_float4(p1.x, p1.y, p1.z, 0.f);
   tri[3 * f + 1] = make_float4(p2.x, p2.y, p2.z, 0.f);
   tri[3 * f + 2] = make_float4(p3.x, p3.y, p3.z, 0.f);
-  nrm[3 * f] = make_float4(nn[0], nn[1], nn[2], 0.f);
-  nrm[3 * f + 1] = make_float4(nn[3], nn[4], nn[5], 0.f);
-  nrm[3 * f + 2] = make_float4(nn[6], nn[7], nn[8], 0.f);
   const V3 c = cross(p2 - p1, p3 - p1);
   const V3 g = normalize(c);
   geo[f] = make_float4(g.x, g.y, g.z, 0.5f * length(c));
+}
+
+// Vertex normals, 3 per face.
+__global__ void normals_kernel(const float* __restrict__ nrms, int n3, float4* __restrict__ nrm) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n3) return;
+  const float* v = nrms + 3 * (size_t)i;
+  nrm[i] = make_float4(v[0], v[1], v[2], 0.f);
+}
+
+void scene_normals_launch(const float* nrms, int n, float4* nrm, cudaStream_t st) {
+  if (n > 0) normals_kernel<<<(3 * n + 255) / 256, 256, 0, st>>>(nrms, 3 * n, nrm);
 }
 
 __global__ void scene_bbox_kernel(const float4* __restrict__ tri, int n,
@@ -116,6 +124,7 @@ __global__ void leaf_setup_kernel(const float4* __restrict__ tri, int n,
 
 constexpr int kPlocRadius = 16;
 constexpr int kPlocBlock = 256;
+constexpr int kPlocMaxBlocks = 4096;
 
 __device__ __forceinline__ float union_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
   const float dx = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x);
@@ -150,93 +159,197 @@ __global__ void ploc_leaf_kernel(const float4* __restrict__ mt, int n,
   cid[leaf] = ~leaf;
 }
 
-// nn[i] = the cluster j != i, |i - j| <= kPlocRadius, whose pair with i
-// comes first in the pair order. m >= 2.
-__global__ void __launch_bounds__(kPlocBlock)
-    ploc_nn_kernel(const float4* __restrict__ blo, const float4* __restrict__ bhi, int m,
-                   int* __restrict__ nn) {
-  __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius];
-  __shared__ float4 shi[kPlocBlock + 2 * kPlocRadius];
-  const int base = blockIdx.x * kPlocBlock - kPlocRadius;
-  for (int t = threadIdx.x; t < kPlocBlock + 2 * kPlocRadius; t += blockDim.x) {
-    const int k = base + t;
-    if (k >= 0 && k < m) {
-      slo[t] = blo[k];
-      shi[t] = bhi[k];
+// All passes in one cooperative launch. Launched pass by pass (9 launches and a
+// read-back each), the 55 passes of 249k triangles took 2.1 ms of kernels and
+// most of the 7.7 ms of an upload with the gaps between them; the clusters left
+// decide the next pass, so the launch waits for itself at grid barriers instead,
+// and once the clusters left fit one block, that block goes on alone: 0.64 ms,
+// 4.8 ms the upload (1.8 ms with the other copies beside it, upload_scene).
+//
+// A pass: block b owns the clusters [b * per, (b + 1) * per).
+//   1. nn[i] = the cluster j != i, |i - j| <= kPlocRadius, whose pair with i
+//      comes first in the pair order;
+//   2. the block counts its merges (mutual pairs i < nn[i], owned by i) and the
+//      clusters it keeps (all but the absorbed ones);
+//   3. the counts of the blocks before it give each owner's node (top - 1 - its
+//      rank among the owners) and each kept cluster's new place.
+
+// Boxes of a tile of clusters and kPlocRadius more on either side.
+struct PlocTile {
+  float4 lo[kPlocBlock + 2 * kPlocRadius];
+  float4 hi[kPlocBlock + 2 * kPlocRadius];
+};
+
+__device__ __forceinline__ void ploc_neighbours(PlocTile& t, const float4* blo, const float4* bhi,
+                                                int m, int first, int last, int* nn) {
+  for (int c0 = first; c0 < last; c0 += kPlocBlock) {
+    const int base = c0 - kPlocRadius;
+    __syncthreads();
+    for (int q = threadIdx.x; q < kPlocBlock + 2 * kPlocRadius; q += kPlocBlock) {
+      const int k = base + q;
+      if (k >= 0 && k < m) {
+        t.lo[q] = blo[k];
+        t.hi[q] = bhi[k];
+      }
     }
-  }
-  __syncthreads();
-  const int i = blockIdx.x * kPlocBlock + threadIdx.x;
-  if (i >= m) return;
-  const float4 lo = slo[threadIdx.x + kPlocRadius], hi = shi[threadIdx.x + kPlocRadius];
-  float best = INFINITY;
-  int bj = -1, bkey = 0;
-  for (int o = -kPlocRadius; o <= kPlocRadius; ++o) {
-    const int j = i + o;
-    if (o == 0 || j < 0 || j >= m) continue;
-    const int t = threadIdx.x + kPlocRadius + o;
-    const float c = union_area(lo, hi, slo[t], shi[t]);
-    // ties: nearer first, then an even smaller index, then the smaller one
-    const int mn = min(i, j);
-    const int key = (abs(o) << 2) | ((mn & 1) << 1) | (o > 0 ? 1 : 0);
-    if (c < best || (c == best && key < bkey)) {
-      best = c;
-      bj = j;
-      bkey = key;
+    __syncthreads();
+    const int i = c0 + threadIdx.x;
+    if (i >= last) continue;
+    const float4 lo = t.lo[threadIdx.x + kPlocRadius], hi = t.hi[threadIdx.x + kPlocRadius];
+    float best = INFINITY;
+    int bj = -1, bkey = 0;
+    for (int o = -kPlocRadius; o <= kPlocRadius; ++o) {
+      const int j = i + o;
+      if (o == 0 || j < 0 || j >= m) continue;
+      const int q = threadIdx.x + kPlocRadius + o;
+      const float c = union_area(lo, hi, t.lo[q], t.hi[q]);
+      // ties: nearer first, then an even smaller index, then the smaller one
+      const int mn = min(i, j);
+      const int key = (abs(o) << 2) | ((mn & 1) << 1) | (o > 0 ? 1 : 0);
+      if (c < best || (c == best && key < bkey)) {
+        best = c;
+        bj = j;
+        bkey = key;
+      }
     }
+    nn[i] = bj;
   }
-  nn[i] = bj;
 }
 
-// mflag[i]: i merges with nn[i] and owns the new node (mutual, i < nn[i]);
-// keep[i]: cluster i survives the pass (not absorbed by a smaller owner).
-__global__ void ploc_flags_kernel(const int* __restrict__ nn, int m, uint32_t* __restrict__ mflag,
-                                  uint32_t* __restrict__ keep) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
+// {merges owned, clusters kept} of cluster i as two 16-bit counts (a block of
+// at most 256 x 255 clusters per scan).
+__device__ __forceinline__ uint32_t ploc_flags(const int* nn, int i) {
   const int j = nn[i];
   const bool mutual = nn[j] == i;
-  mflag[i] = mutual && i < j;
-  keep[i] = !(mutual && j < i);
+  return (mutual && i < j ? 1u : 0u) | (mutual && j < i ? 0u : 0x10000u);
 }
 
-// The pass's merges and the compacted clusters. Merge owner i gets node
-// top - 1 - mrank[i]; out[0] = clusters left, out[1] = merges.
-__global__ void ploc_merge_kernel(const int* __restrict__ cid, const float4* __restrict__ blo,
-                                  const float4* __restrict__ bhi, const int* __restrict__ nn,
-                                  int m, const uint32_t* __restrict__ mflag,
-                                  const uint32_t* __restrict__ mrank,
-                                  const uint32_t* __restrict__ keep,
-                                  const uint32_t* __restrict__ kpos, int top,
-                                  int* __restrict__ cid2, float4* __restrict__ blo2,
-                                  float4* __restrict__ bhi2, float4* __restrict__ nodes,
-                                  int* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  if (i == m - 1) {
-    out[0] = (int)(kpos[i] + keep[i]);
-    out[1] = (int)(mrank[i] + mflag[i]);
+// Merges and compacts the clusters [first, last); `merged` owners and `kept`
+// clusters lie before them.
+__device__ __forceinline__ void ploc_merge(const int* cid, const float4* blo, const float4* bhi,
+                                           const int* nn, int first, int last, int merged, int kept,
+                                           int top, int* cid2, float4* blo2, float4* bhi2,
+                                           float4* nodes, uint32_t* ws) {
+  for (int c0 = first; c0 < last; c0 += kPlocBlock) {
+    const int i = c0 + threadIdx.x;
+    const uint32_t f = i < last ? ploc_flags(nn, i) : 0u;
+    uint32_t total;
+    const uint32_t before = block_exclusive_scan(f, ws, &total);
+    if (f >> 16) {
+      const float4 alo = blo[i], ahi = bhi[i];
+      const int o = kept + (int)(before >> 16);
+      if (!(f & 1u)) {
+        cid2[o] = cid[i];
+        blo2[o] = alo;
+        bhi2[o] = ahi;
+      } else {
+        const int j = nn[i];
+        const float4 clo = blo[j], chi = bhi[j];
+        const int idx = top - 1 - (merged + (int)(before & 0xffffu));
+        float4* nd = nodes + 4 * (size_t)idx;
+        nd[0] = make_float4(alo.x, alo.y, alo.z, __int_as_float(cid[i]));
+        nd[1] = make_float4(ahi.x, ahi.y, ahi.z, __int_as_float(cid[j]));
+        nd[2] = make_float4(clo.x, clo.y, clo.z, 0.f);
+        nd[3] = make_float4(chi.x, chi.y, chi.z, 0.f);
+        cid2[o] = idx;
+        blo2[o] = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), 0.f);
+        bhi2[o] = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
+      }
+    }
+    merged += (int)(total & 0xffffu);
+    kept += (int)(total >> 16);
   }
-  if (!keep[i]) return;
-  const float4 alo = blo[i], ahi = bhi[i];
-  const int o = (int)kpos[i];
-  if (!mflag[i]) {
-    cid2[o] = cid[i];
-    blo2[o] = alo;
-    bhi2[o] = ahi;
-    return;
+}
+
+// Clusters left that one block takes alone (16 rounds of its threads).
+constexpr int kPlocAlone = 16 * kPlocBlock;
+
+__global__ void __launch_bounds__(kPlocBlock)
+    ploc_kernel(int* cid_a, float4* blo_a, float4* bhi_a, int* cid_b, float4* blo_b, float4* bhi_b,
+                int* nn, int n, float4* nodes, int2* counts, int* left) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  __shared__ PlocTile tile;
+  __shared__ uint32_t ws[kPlocBlock / 32];
+  __shared__ int2 sum;
+  int m = n, top = n - 1;
+  // every pass merges at least one pair: at most n - 1 passes
+  for (int pass = 0; m > 1 && pass < n; ++pass) {
+    const bool alone = m <= kPlocAlone;
+    if (alone && blockIdx.x != 0) return;
+    const int per = alone ? m : (m + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int first = min((int)blockIdx.x * per, m), last = min(first + per, m);
+    ploc_neighbours(tile, blo_a, bhi_a, m, first, last, nn);
+    if (alone) __syncthreads();
+    else grid.sync();
+    int2 mine = make_int2(0, 0);
+    for (int i = first + threadIdx.x; i < last; i += kPlocBlock) {
+      const uint32_t f = ploc_flags(nn, i);
+      mine.x += (int)(f & 1u);
+      mine.y += (int)(f >> 16);
+    }
+    if (threadIdx.x == 0) sum = make_int2(0, 0);
+    __syncthreads();
+    mine.x = __reduce_add_sync(kFull, mine.x);
+    mine.y = __reduce_add_sync(kFull, mine.y);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&sum.x, mine.x);
+      atomicAdd(&sum.y, mine.y);
+    }
+    __syncthreads();
+    int2 before = make_int2(0, 0), all = sum;
+    if (!alone) {
+      if (threadIdx.x == 0) counts[blockIdx.x] = sum;
+      grid.sync();
+      // every block adds up all blocks' counts
+      int2 b = make_int2(0, 0), t = make_int2(0, 0);
+      for (int q = threadIdx.x; q < (int)gridDim.x; q += kPlocBlock) {
+        const int2 c = counts[q];
+        t.x += c.x;
+        t.y += c.y;
+        if (q < (int)blockIdx.x) {
+          b.x += c.x;
+          b.y += c.y;
+        }
+      }
+      __shared__ int tot[4];
+      if (threadIdx.x < 4) tot[threadIdx.x] = 0;
+      __syncthreads();
+      b.x = __reduce_add_sync(kFull, b.x);
+      b.y = __reduce_add_sync(kFull, b.y);
+      t.x = __reduce_add_sync(kFull, t.x);
+      t.y = __reduce_add_sync(kFull, t.y);
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&tot[0], b.x);
+        atomicAdd(&tot[1], b.y);
+        atomicAdd(&tot[2], t.x);
+        atomicAdd(&tot[3], t.y);
+      }
+      __syncthreads();
+      before = make_int2(tot[0], tot[1]);
+      all = make_int2(tot[2], tot[3]);
+    }
+    // every block sees the same counts, so all end together
+    if (all.x < 1 || all.x > top || all.y != m - all.x) break;  // cannot happen with the tie rule
+    ploc_merge(cid_a, blo_a, bhi_a, nn, first, last, before.x, before.y, top, cid_b, blo_b, bhi_b,
+               nodes, ws);
+    if (alone) __syncthreads();
+    else grid.sync();
+    m = all.y;
+    top -= all.x;
+    int* ci = cid_a;
+    cid_a = cid_b;
+    cid_b = ci;
+    float4* f = blo_a;
+    blo_a = blo_b;
+    blo_b = f;
+    f = bhi_a;
+    bhi_a = bhi_b;
+    bhi_b = f;
   }
-  const int j = nn[i];
-  const float4 clo = blo[j], chi = bhi[j];
-  const int idx = top - 1 - (int)mrank[i];
-  float4* nd = nodes + 4 * (size_t)idx;
-  nd[0] = make_float4(alo.x, alo.y, alo.z, __int_as_float(cid[i]));
-  nd[1] = make_float4(ahi.x, ahi.y, ahi.z, __int_as_float(cid[j]));
-  nd[2] = make_float4(clo.x, clo.y, clo.z, 0.f);
-  nd[3] = make_float4(chi.x, chi.y, chi.z, 0.f);
-  cid2[o] = idx;
-  blo2[o] = make_float4(fminf(alo.x, clo.x), fminf(alo.y, clo.y), fminf(alo.z, clo.z), 0.f);
-  bhi2[o] = make_float4(fmaxf(ahi.x, chi.x), fmaxf(ahi.y, chi.y), fmaxf(ahi.z, chi.z), 0.f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    left[0] = m;
+    left[1] = top;
+  }
 }
 
 // Record i of the tree that walks use (pm_scene.cuh) from the binary nodes
@@ -290,19 +403,25 @@ __global__ void widen_kernel(const float4* __restrict__ binary, int n, float4* _
   w[7] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-size_t scene_build_scratch_bytes(int n) {
-  const size_t nn = (size_t)(n > 1 ? n : 2);
-  // cluster boxes a/b (4n float4), sort keys / values a/b (4n), histogram,
-  // scene box, cluster ids a/b and neighbours (3n), pass flags and ranks
-  // (4n), scan tile sums, pass counts
-  // and the binary nodes (4n float4)
-  return 4 * nn * 16 + 4 * nn * 16 + 4 * nn * 4 + sort_hist_words(nn) * 4 + 64 + 3 * nn * 4 + 4 * nn * 4 +
-         (size_t)scan_tiles((int64_t)nn) * 4 + 64;
+static float host_from_ordered(uint32_t u) {
+  u = (u & 0x80000000u) ? (u & 0x7fffffffu) : ~u;
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
 }
 
-cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, float4* tri,
-                               float4* nrm, float4* geo, float4* mt, float4* wide,
-                               void* scratch, cudaStream_t st) {
+size_t scene_build_scratch_bytes(int n) {
+  const size_t nn = (size_t)(n > 1 ? n : 2);
+  // cluster boxes a/b (4n float4), the binary nodes (4n float4), sort keys /
+  // values a/b (4n), histogram, scene box, cluster ids a/b and neighbours (3n),
+  // clusters left, and the counts of up to kPlocMaxBlocks blocks
+  return 4 * nn * 16 + 4 * nn * 16 + 4 * nn * 4 + sort_hist_words(nn) * 4 + 64 + 3 * nn * 4 + 32 +
+         kPlocMaxBlocks * sizeof(int2) + 64;
+}
+
+cudaError_t scene_build_launch(const float* verts, int n, float4* tri, float4* geo, float4* mt,
+                               float4* wide, void* scratch, SceneBuildResult* result,
+                               cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   float4* blo_a = (float4*)scratch;
   float4* bhi_a = blo_a + n;
@@ -318,17 +437,14 @@ cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, flo
   int* cid_a = (int*)(bb + 16);
   int* cid_b = cid_a + n;
   int* nn = cid_b + n;
-  uint32_t* mflag = (uint32_t*)(nn + n);
-  uint32_t* keep = mflag + n;
-  uint32_t* mrank = keep + n;
-  uint32_t* kpos = mrank + n;
-  uint32_t* sums = kpos + n;
-  int* out = (int*)(sums + scan_tiles(n));
+  int* out = (int*)bb + 8;
+  int2* counts = (int2*)(((uintptr_t)(nn + n) + 15) & ~(uintptr_t)15);
   const int tb = 256;
   const int gb = (n + tb - 1) / tb;
-  face_setup_kernel<<<gb, tb, 0, st>>>(verts, nrms, n, tri, nrm, geo);
+  *result = SceneBuildResult{bb};
+  face_setup_kernel<<<gb, tb, 0, st>>>(verts, n, tri, geo);
   cudaMemsetAsync(bb, 0xff, 3 * sizeof(uint32_t), st);
-  cudaMemsetAsync(bb + 3, 0x00, 3 * sizeof(uint32_t), st);
+  cudaMemsetAsync(bb + 3, 0x00, 13 * sizeof(uint32_t), st);
   scene_bbox_kernel<<<min(gb, 1184), tb, 0, st>>>(tri, n, bb);
   tri_morton_kernel<<<gb, tb, 0, st>>>(tri, n, bb, ka, va);
   const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, n, 30, hist, st);
@@ -336,33 +452,27 @@ cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, flo
   leaf_setup_kernel<<<gb, tb, 0, st>>>(tri, n, order, mt);
   if (n == 1) return cudaGetLastError();
   ploc_leaf_kernel<<<gb, tb, 0, st>>>(mt, n, bb, cid_a, blo_a, bhi_a);
-  int m = n, top = n - 1;
-  int counts[2] = {0, 0};
-  cudaError_t e;
-  // every pass merges at least one pair: at most n - 1 passes
-  for (int pass = 0; m > 1 && pass < n; ++pass) {
-    const int g = (m + tb - 1) / tb;
-    ploc_nn_kernel<<<(m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(blo_a, bhi_a, m,
-                                                                             nn);
-    ploc_flags_kernel<<<g, tb, 0, st>>>(nn, m, mflag, keep);
-    exclusive_scan_u32(mflag, mrank, m, sums, st);
-    exclusive_scan_u32(keep, kpos, m, sums, st);
-    ploc_merge_kernel<<<g, tb, 0, st>>>(cid_a, blo_a, bhi_a, nn, m, mflag, mrank, keep, kpos, top,
-                                        cid_b, blo_b, bhi_b, nodes, out);
-    if ((e = cudaMemcpyAsync(counts, out, sizeof(counts), cudaMemcpyDeviceToHost, st)) ||
-        (e = cudaStreamSynchronize(st)))
-      return e;
-    if (counts[1] < 1 || counts[1] > top || counts[0] != m - counts[1])
-      return cudaErrorUnknown;  // no progress: cannot happen with the tie rule
-    m = counts[0];
-    top -= counts[1];
-    std::swap(cid_a, cid_b);
-    std::swap(blo_a, blo_b);
-    std::swap(bhi_a, bhi_b);
-  }
-  if (m != 1 || top != 0) return cudaErrorUnknown;
+  int dev = 0, sms = 148, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ploc_kernel, kPlocBlock, 0);
+  if (e != cudaSuccess) return e;
+  int blocks = std::min((n + kPlocBlock - 1) / kPlocBlock, sms * std::max(1, std::min(per_sm, 4)));
+  blocks = std::min(blocks, kPlocMaxBlocks);
+  if (n <= kPlocAlone) blocks = 1;
+  void* args[] = {&cid_a, &blo_a, &bhi_a, &cid_b, &blo_b, &bhi_b, &nn, &n, &nodes, &counts, &out};
+  if ((e = cudaLaunchCooperativeKernel((const void*)ploc_kernel, blocks, kPlocBlock, args, 0, st)))
+    return e;
   widen_kernel<<<(n - 1 + tb - 1) / tb, tb, 0, st>>>(nodes, n - 1, wide);
   return cudaGetLastError();
+}
+
+bool SceneBuildResult::read(const uint32_t host[16], int n, float lo[3], float hi[3]) {
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = host_from_ordered(host[a]);
+    hi[a] = host_from_ordered(host[3 + a]);
+  }
+  return n == 1 || (host[8] == 1u && host[9] == 0u);
 }
 
 // Batched closest-hit queries (Scene::intersect, scene.h:307-348).

@@ -8,12 +8,22 @@ namespace pm {
 // Scratch bytes scene_build_launch needs for n faces.
 size_t scene_build_scratch_bytes(int n);
 
-// verts / nrms: device, 9 floats per face. Fills tri, nrm, geo (face
-// order), mt (leaf order) and nodes (n - 1 records of 8 float4). Synchronises st
-// once per clustering pass (it reads the clusters left).
-cudaError_t scene_build_launch(const float* verts, const float* nrms, int n, float4* tri,
-                               float4* nrm, float4* geo, float4* mt, float4* nodes,
-                               void* scratch, cudaStream_t st);
+// What a build leaves in its scratch: 16 words to be read back once the stream
+// has reached them.
+struct SceneBuildResult {
+  const uint32_t* words;
+  // The vertices' bounds; false when the tree was not completed.
+  static bool read(const uint32_t host[16], int n, float lo[3], float hi[3]);
+};
+
+// verts: device, 9 floats per face. Fills tri, geo (face order), mt (leaf
+// order) and nodes (n - 1 records of 8 float4). Does not synchronise.
+cudaError_t scene_build_launch(const float* verts, int n, float4* tri, float4* geo, float4* mt,
+                               float4* nodes, void* scratch, SceneBuildResult* result,
+                               cudaStream_t st);
+
+// nrms: device, 9 floats per face; nrm: 3 float4 per face.
+void scene_normals_launch(const float* nrms, int n, float4* nrm, cudaStream_t st);
 
 // rays: 2 float4 per ray {origin, tmin}, {direction, tmax}; out: one float4
 // per ray {t, u, v, face id bits (-1: miss)}.
