@@ -160,15 +160,15 @@ int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq,
   const MapDev m = map_view(dm);
   query_keys_launch(m, d_q, nq, 3, ka, va, st);
   const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, (int)nq, kQueryKeyBits, hist, st);
-  // the keys' place is free again: the list of the queries left
-  const TileDefer left{ka, hist, false};
+  // the keys' places are free again: the list of the queries left
+  const TileDefer left{ka, (float*)kb, hist, false};
   cudaError_t e = knn_tile_launch(m, d_q, nq, k, n_emitted, d_rgb, left, c->next_counter(),
                                   c->num_sms, st, in_b ? vb : va, 3);
   if (e == cudaSuccess) {
     KnnOut o{};
     o.rgb = d_rgb;
     e = knn_launch(m, d_q, nq, k, kModeRadiance, n_emitted, o, c->next_counter(), c->num_sms, st,
-                   ka, 3, hist);
+                   ka, 3, hist, left.tau);
   }
   const cudaError_t e2 = cudaEventRecord(sc->done, st);
   return cuda_status(c, e != cudaSuccess ? e : e2, "radiance launch");

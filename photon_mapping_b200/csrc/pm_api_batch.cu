@@ -364,21 +364,23 @@ cudaError_t enqueue_knn(pm_batch* b, const uint32_t* order, const pm_batch_tunin
   int64_t max_items = b->nq / chunk + b->n;
   unsigned long long* counter = (unsigned long long*)b->knn_counter.ptr;
   uint32_t *left = nullptr, *left_n = nullptr;
+  float* left_tau = nullptr;
   if (b->tiles) {
     // the unsorted keys' place is free
     left = (uint32_t*)(b->sorted_in_b ? b->qka.ptr : b->qkb.ptr);
+    left_tau = (float*)(left + b->nq);
     left_n = (uint32_t*)(counter + 2);
     const cudaError_t e = batch_tile_launch(
         b->tables, (const float4*)b->slots.ptr, order, (const int64_t*)b->qoff.ptr,
         (const int64_t*)b->item_off.ptr, max_items, chunk, b->max_k, (float*)b->res.ptr, left,
-        left_n, b->tile_per_sm, counter + 1, b->num_sms, b->st);
+        left_tau, left_n, b->tile_per_sm, counter + 1, b->num_sms, b->st);
     if (e != cudaSuccess) return e;
     max_items = b->nq;
   }
   return batch_knn_launch(b->tables, (const float4*)b->slots.ptr, order,
                           (const int64_t*)b->qoff.ptr, (const int64_t*)b->item_off.ptr,
                           max_items, (float*)b->res.ptr, t.knn_warps, t.knn_chunk, t.knn_buffer,
-                          per_sm, counter, b->num_sms, b->st, left, left_n);
+                          per_sm, counter, b->num_sms, b->st, left, left_tau, left_n);
 }
 
 // The whole step with the current tuning (no host synchronisation).

@@ -38,40 +38,43 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
                    bool need_caustics, int kg, int kc, int64_t* q_tot,
                    const float* slot_adj, float4* const* photon_adj) {
   cudaStream_t st = c->stream;
-  uint32_t* ka = (uint32_t*)c->r_sort.ptr;
-  uint32_t* kb = ka + n_slots;
-  uint32_t* va = kb + n_slots;
-  uint32_t* vb = va + n_slots;
-  uint32_t* hist = vb + n_slots;
+  uint32_t* const keys_a = (uint32_t*)c->r_sort.ptr;
+  uint32_t* const keys_b = keys_a + n_slots;
+  uint32_t* const vals_a = keys_b + n_slots;
+  uint32_t* const vals_b = vals_a + n_slots;
+  uint32_t* hist = vals_b + n_slots;
   unsigned* qcount = (unsigned*)((char*)c->r_misc.ptr + 16);
+  unsigned nqs[2] = {0, 0};
   cudaError_t e;
+  if ((e = cudaMemsetAsync(qcount, 0, 8, st)) != cudaSuccess) return cuda_status(c, e, "render");
+  render_list_queries(a.slots, a.sample_rec, ns, n_slots, a.q_per_sample, c->scene.lo, c->scene.hi,
+                      keys_a, vals_a, qcount, st);
+  if ((e = cudaMemcpyAsync(nqs, qcount, 8, cudaMemcpyDeviceToHost, st)) ||
+      (e = cudaStreamSynchronize(st)))
+    return cuda_status(c, e, "render queries");
   for (int map = 0; map < 2; ++map) {
     if (map == 1 && !need_caustics) continue;
-    if ((e = cudaMemsetAsync(qcount, 0, 4, st)) != cudaSuccess)
-      return cuda_status(c, e, "render");
-    render_list_queries(a.slots, a.sample_rec, ns, a.q_per_sample, map, c->scene.lo,
-                        c->scene.hi, ka, va, qcount, st);
-    unsigned nq = 0;
-    if ((e = cudaMemcpyAsync(&nq, qcount, 4, cudaMemcpyDeviceToHost, st)) ||
-        (e = cudaStreamSynchronize(st)))
-      return cuda_status(c, e, "render queries");
+    const unsigned nq = nqs[map];
     q_tot[map] += nq;
     if (nq == 0) continue;
+    // the caustics map's list lies at the end
+    const size_t at = map == 0 ? 0 : (size_t)n_slots - nq;
+    uint32_t *ka = keys_a + at, *kb = keys_b + at, *va = vals_a + at, *vb = vals_b + at;
     const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, (int)nq, 30, hist, st);
     KnnOut o{};
     o.rgb = (float*)c->r_res.ptr;
     o.stats = c->stats_ptr();
     if (!slot_adj && use_tiles(c, c->maps[map], nq, map == 0 ? kg : kc, true)) {
-      // the sorted keys' place is free: the list of the queries the tiles leave
+      // the sorted keys' places are free: the list of the queries the tiles leave
       uint32_t* left_n = (uint32_t*)((char*)c->r_misc.ptr + 56);
-      const TileDefer left{ka, left_n, false};
+      const TileDefer left{ka, (float*)kb, left_n, false};
       const MapDev m = map_view(c->maps[map]);
       const int k = map == 0 ? kg : kc;
       e = knn_tile_launch(m, a.slots, nq, k, (float)c->map_emitted[map], o.rgb, left,
                           c->next_counter(), c->num_sms, st, in_b ? vb : va, 4);
       if (e == cudaSuccess)
         e = knn_launch(m, a.slots, nq, k, kModeRadiance, (float)c->map_emitted[map], o,
-                       c->next_counter(), c->num_sms, st, ka, 4, left_n);
+                       c->next_counter(), c->num_sms, st, ka, 4, left_n, left.tau);
       if (e != cudaSuccess) return cuda_status(c, e, "render estimates");
       continue;
     }

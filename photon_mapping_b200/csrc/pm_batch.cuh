@@ -134,22 +134,25 @@ void batch_query_ranges_launch(const unsigned long long* sorted_keys, int64_t nq
 // batch_knn_prepare sets the kernel's shared-memory limit and gives its
 // resident blocks per SM; call it before capturing a launch in a graph.
 // left: when not null, only the queries at the sorted places left[0 .. *left_n)
-// are answered, one per work item (item_off and chunk unused).
+// are answered, one per work item (item_off and chunk unused), trying the squared
+// radius left_tau of each first.
 cudaError_t batch_knn_prepare(int warps, int buffer, int* blocks_per_sm);
 cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
                              const int64_t* qoff, const int64_t* item_off, int64_t max_items,
                              float* res, int warps, int chunk, int buffer, int blocks_per_sm,
                              unsigned long long* counter, int num_sms, cudaStream_t st,
-                             const uint32_t* left = nullptr, const uint32_t* left_n = nullptr);
+                             const uint32_t* left = nullptr, const float* left_tau = nullptr,
+                             const uint32_t* left_n = nullptr);
 
 // The same by tiles of sorted queries (pm_knn_tile.cu; every k <= kTileMaxK):
 // work items of batch_tile_item() queries, item_off counting those; the queries
-// that tiles leave go to left / left_n. batch_tile_prepare as above.
+// that tiles leave go to left / left_tau / left_n. batch_tile_prepare as above.
 int batch_tile_item(int64_t nq, int num_sms);
 cudaError_t batch_tile_prepare(int max_k, int* blocks_per_sm);
 cudaError_t batch_tile_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
                               const int64_t* qoff, const int64_t* item_off, int64_t max_items,
-                              int item, int max_k, float* res, uint32_t* left, uint32_t* left_n,
+                              int item, int max_k, float* res, uint32_t* left, float* left_tau,
+                              uint32_t* left_n,
                               int blocks_per_sm, unsigned long long* counter, int num_sms,
                               cudaStream_t st);
 

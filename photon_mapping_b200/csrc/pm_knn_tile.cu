@@ -234,6 +234,13 @@ __device__ __forceinline__ void tile_bins(const F2 px[4], const F2 py[4], const 
   w1 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
 }
 
+// Leaves a query to the warp-per-query kernel, with a radius to try.
+__device__ __forceinline__ void leave(const TileDefer& defer, uint32_t query, float tau) {
+  const uint32_t o = atomicAdd(defer.count, 1u);
+  defer.list[o] = query;
+  defer.tau[o] = tau;
+}
+
 // Queries [q0, q0 + nq) (nq <= 32) in the order of `order`. tau: the squared
 // search radius to try first (in/out).
 __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, TileWarp& s, int rows,
@@ -259,17 +266,12 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
   const bool bad = isnan(px) || isnan(py) || isnan(pz);
   if (lane < nq && bad) rgb[3 * (size_t)rec] = rgb[3 * (size_t)rec + 1] = rgb[3 * (size_t)rec + 2] = 0.f;
   unsigned todo = __ballot_sync(kFull, lane < nq && !bad);
-  unsigned give_up = 0;  // queries left to the warp-per-query kernel
   float good = tau;      // from the last queries answered
   int span = kTileQ, sq = kSubQ, tries = 0;
   while (todo) {
-    if (++tries > kTries) {
-      give_up |= todo;
-      break;
-    }
     const float tw = tau * kWalkSlack;
-    if (!(tw > 1e-30f && tw < 1e30f)) {
-      give_up |= todo;
+    if (++tries > kTries || !(tw > 1e-30f && tw < 1e30f)) {
+      if ((todo >> lane) & 1u) leave(defer, defer.positions ? (uint32_t)(q0 + lane) : rec, tau);
       break;
     }
     unsigned wm = near_run(todo, span, kWalkReach * tau, px, py, pz, lane);
@@ -589,11 +591,9 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
       const uint32_t kth = fit ? s.kth[qs] : 0u;
       if (fit && h < 3)
         rgb[3 * (size_t)rq + h] = radiance_from_sum(v, rho, cos_o, n_emitted, __uint_as_float(kth));
-      const unsigned over = __ballot_sync(kFull, act && !fit && h == 0);
-      if (over) {  // bit kLanesQ q: query q of the sub-tile
-        for (int q = 0; q < ns; ++q)
-          if ((over >> (kLanesQ * q)) & 1u) give_up |= 1u << s.ql[q];
-      }
+      if (act && !fit && h == 0)  // the radius up to byte hi holds k photons
+        leave(defer, defer.positions ? (uint32_t)(q0 + s.ql[qs]) : rq,
+              tf * (float)hi * (1.01f / (float)kBins));
       todo &= ~sm;
       wm &= ~sm;
       const uint32_t far = __reduce_max_sync(kFull, kth);
@@ -606,14 +606,6 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
     if (span < kTileQ && !wm) span <<= 1;
   }
   tau = good;
-  if (give_up) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(defer.count, (uint32_t)__popc(give_up));
-    base = __shfl_sync(kFull, base, 0);
-    if ((give_up >> lane) & 1u)
-      defer.list[base + __popc(give_up & lt_mask(lane))] =
-          defer.positions ? (uint32_t)(q0 + lane) : rec;
-  }
 }
 
 // 8 bits per axis separate the queries of a frame as finely as tiles of 32 need.
@@ -711,7 +703,10 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(defer.count, (uint32_t)nq);
       base = __shfl_sync(kFull, base, 0);
-      if (lane < nq) defer.list[base + lane] = (uint32_t)(q0 + lane);
+      if (lane < nq) {
+        defer.list[base + lane] = (uint32_t)(q0 + lane);
+        defer.tau[base + lane] = 0.f;
+      }
       continue;
     }
     tile_item(wmap[warp], wlev[warp], s, rows, lane, slots, order, 4, q0, nq, k, n_emitted, rgb,
@@ -789,7 +784,7 @@ cudaError_t batch_tile_prepare(int max_k, int* blocks_per_sm) {
 
 cudaError_t batch_tile_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
                               const int64_t* qoff, const int64_t* item_off, int64_t max_items,
-                              int item, int max_k, float* res, uint32_t* left, uint32_t* left_n,
+                              int item, int max_k, float* res, uint32_t* left, float* left_tau, uint32_t* left_n,
                               int blocks_per_sm, unsigned long long* counter, int num_sms,
                               cudaStream_t st) {
   const int rows = tile_rows(max_k);
@@ -801,7 +796,7 @@ cudaError_t batch_tile_launch(const BatchTables& t, const float4* slots, const u
       (e = cudaMemsetAsync(left_n, 0, sizeof(uint32_t), st)) != cudaSuccess)
     return e;
   knn_tile_batch_kernel<<<(unsigned)blocks, 32 * kTileWarps, kTileWarps * tile_bytes(rows), st>>>(
-      t, slots, order, qoff, item_off, item, res, rows, TileDefer{left, left_n, true}, counter);
+      t, slots, order, qoff, item_off, item, res, rows, TileDefer{left, left_tau, left_n, true}, counter);
   return cudaGetLastError();
 }
 

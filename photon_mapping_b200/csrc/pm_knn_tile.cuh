@@ -15,6 +15,7 @@ struct TileLevels {
 // places in the sorted order), and how many.
 struct TileDefer {
   uint32_t* list;
+  float* tau;  // a squared radius to try for each of them (0: none known)
   uint32_t* count;
   bool positions;
 };

@@ -818,7 +818,8 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
                                           int lane, const void* __restrict__ queries,
                                           int64_t qb, int64_t qe, int k, float n_emitted,
                                           const KnnOut& out, const uint32_t* __restrict__ order,
-                                          int stride4, float& r_hint, bool grouped = true) {
+                                          int stride4, float& r_hint, bool grouped = true,
+                                          const float* __restrict__ taus = nullptr) {
   const float kInf = __int_as_float(0x7f800000);
   bool have_prev = false;
   float pqx = 0.f, pqy = 0.f, pqz = 0.f, pkth = 0.f;
@@ -894,7 +895,9 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       if (!warm) {
         stat_add<S>(s, lane, kStatCold, 1);
         guess = true;
-        tg = r_hint > 0.f ? 1.69f * r_hint * r_hint : even_tau(m, L.oc[m.nlevels - 1].x, k);
+        tg = taus ? __ldg(taus + qi) : 0.f;
+        if (!(tg > 0.f))
+          tg = r_hint > 0.f ? 1.69f * r_hint * r_hint : even_tau(m, L.oc[m.nlevels - 1].x, k);
         if (!(tg > 1e-37f)) tg = 1e-37f;  // NaN too
         q.tau = tg;
       }
@@ -1040,7 +1043,7 @@ __global__ void __launch_bounds__(256, 4)
                float n_emitted, KnnOut out,
                unsigned long long* __restrict__ counter,
                const uint32_t* __restrict__ order, int stride4,
-               const uint32_t* __restrict__ nq_dev) {
+               const uint32_t* __restrict__ nq_dev, const float* __restrict__ taus) {
   if (nq_dev) {
     nq = (int64_t)*nq_dev;
     if (nq == 0) return;
@@ -1076,7 +1079,7 @@ __global__ void __launch_bounds__(256, 4)
     const int64_t qe = min(nq, qb + (head ? kChunk : tail));
 
     knn_chunk<C, MODE, S, true>(m, L, s, lane, queries, qb, qe, k, n_emitted, out, order, stride4,
-                                r_hint, tail == kTail);
+                                r_hint, tail == kTail, taus);
     if (S) {
       __syncwarp();
       if (lane < kNumStats) {
@@ -1093,7 +1096,7 @@ static cudaError_t launch_one(const MapDev& m, const void* queries,
                               int64_t nq, int k, float n_emitted, KnnOut out,
                               unsigned long long* counter, int num_sms,
                               cudaStream_t st, const uint32_t* order,
-                              int stride4, const uint32_t* nq_dev) {
+                              int stride4, const uint32_t* nq_dev, const float* taus) {
   constexpr int kThreads = (C <= 512) ? 256 : 128;
   const size_t smem = (kThreads / 32) * sizeof(WarpBuf<C>);
   auto kern = out.stats ? knn_kernel<C, MODE, true> : knn_kernel<C, MODE, false>;
@@ -1113,7 +1116,7 @@ static cudaError_t launch_one(const MapDev& m, const void* queries,
   e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)blocks, kThreads, smem, st>>>(m, queries, nq, k, n_emitted,
-                                                 out, counter, order, stride4, nq_dev);
+                                                 out, counter, order, stride4, nq_dev, taus);
   return cudaGetLastError();
 }
 
@@ -1121,26 +1124,26 @@ cudaError_t knn_launch(const MapDev& m, const void* queries, int64_t nq,
                        int k, int mode, float n_emitted, KnnOut out,
                        unsigned long long* counter, int num_sms,
                        cudaStream_t st, const uint32_t* order, int stride4,
-                       const uint32_t* nq_dev) {
+                       const uint32_t* nq_dev, const float* taus) {
   if (nq <= 0) return cudaSuccess;
   if (mode == kModeAdjoint) {
     return k <= 224 ? launch_one<512, kModeAdjoint>(m, queries, nq, k, n_emitted, out, counter,
-                                                   num_sms, st, order, stride4, nq_dev)
+                                                   num_sms, st, order, stride4, nq_dev, taus)
                     : launch_one<2048, kModeAdjoint>(m, queries, nq, k, n_emitted, out, counter,
-                                                    num_sms, st, order, stride4, nq_dev);
+                                                    num_sms, st, order, stride4, nq_dev, taus);
   }
   if (k <= 224) {
     return mode == kModeRadiance
                ? launch_one<512, kModeRadiance>(m, queries, nq, k, n_emitted,
-                                                out, counter, num_sms, st, order, stride4, nq_dev)
+                                                out, counter, num_sms, st, order, stride4, nq_dev, taus)
                : launch_one<512, kModeKnn>(m, queries, nq, k, n_emitted, out,
-                                           counter, num_sms, st, order, stride4, nq_dev);
+                                           counter, num_sms, st, order, stride4, nq_dev, taus);
   }
   return mode == kModeRadiance
              ? launch_one<2048, kModeRadiance>(m, queries, nq, k, n_emitted,
-                                               out, counter, num_sms, st, order, stride4, nq_dev)
+                                               out, counter, num_sms, st, order, stride4, nq_dev, taus)
              : launch_one<2048, kModeKnn>(m, queries, nq, k, n_emitted, out,
-                                          counter, num_sms, st, order, stride4, nq_dev);
+                                          counter, num_sms, st, order, stride4, nq_dev, taus);
 }
 
 }  // namespace pm
@@ -1159,7 +1162,7 @@ __global__ void __launch_bounds__(256, 4)
                      const uint32_t* __restrict__ order, const int64_t* __restrict__ qoff,
                      const int64_t* __restrict__ item_off, int chunk, KnnOut out,
                      unsigned long long* __restrict__ counter, const uint32_t* __restrict__ left,
-                     const uint32_t* __restrict__ left_n) {
+                     const float* __restrict__ left_tau, const uint32_t* __restrict__ left_n) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int64_t ioff[kMaxBatchScenes + 1];
   __shared__ MapDev wmap[8];
@@ -1196,8 +1199,10 @@ __global__ void __launch_bounds__(256, 4)
     }
     const int64_t qb = left ? at : qoff[sc] + (at - ioff[sc]) * chunk;
     const int64_t qe = left ? at + 1 : min(qoff[sc + 1], qb + chunk);
+    // knn_chunk reads the radius of query qb, so the array starts c0 - qb away
     knn_chunk<C, kModeRadiance, false, false>(wmap[warp], wlev[warp], s, lane, slots, qb, qe, k,
-                                       n_emitted, out, order, 4, r_hint);
+                                              n_emitted, out, order, 4, r_hint, true,
+                                              left ? left_tau + (int64_t)c0 - qb : nullptr);
   }
 }
 
@@ -1219,7 +1224,7 @@ cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const ui
                              const int64_t* qoff, const int64_t* item_off, int64_t max_items,
                              float* res, int warps, int chunk, int buffer, int blocks_per_sm,
                              unsigned long long* counter, int num_sms, cudaStream_t st,
-                             const uint32_t* left, const uint32_t* left_n) {
+                             const uint32_t* left, const float* left_tau, const uint32_t* left_n) {
   if (warps < 1 || warps > 8 || chunk < 1) return cudaErrorInvalidValue;
   const int threads = 32 * warps;
   auto kern = buffer <= 512 ? knn_batch_kernel<512> : knn_batch_kernel<2048>;
@@ -1234,7 +1239,7 @@ cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const ui
   KnnOut out{};
   out.rgb = res;
   kern<<<(unsigned)blocks, threads, smem, st>>>(t, slots, order, qoff, item_off, chunk, out,
-                                                counter, left, left_n);
+                                                counter, left, left_tau, left_n);
   return cudaGetLastError();
 }
 

@@ -93,6 +93,8 @@ struct KnnOut {
 //                  pm_radiance_query at queries + stride4 * r float4s, and
 //                  writes rgb[3r .. 3r+3)
 //   knn mode:      queries = 3 floats per query (order and stride unused)
+//   taus:          with `order`, when not null: a squared radius to try first for
+//                  query i (0: none)
 //   nq_dev:        when not null, the number of queries (at most nq) is read
 //                  from this device word
 //   adjoint mode:  the records of radiance mode; the neighbours of record r
@@ -103,6 +105,7 @@ cudaError_t knn_launch(const MapDev& m, const void* queries, int64_t nq,
                        int k, int mode, float n_emitted, KnnOut out,
                        unsigned long long* counter, int num_sms,
                        cudaStream_t st, const uint32_t* order = nullptr,
-                       int stride4 = 3, const uint32_t* nq_dev = nullptr);
+                       int stride4 = 3, const uint32_t* nq_dev = nullptr,
+                       const float* taus = nullptr);
 
 }  // namespace pm

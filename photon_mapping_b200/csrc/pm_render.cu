@@ -230,44 +230,74 @@ __global__ void rng_init_kernel(unsigned long long* st, int w, int n) {
   st[p] = (unsigned long long)(j + w * i);  // UniformSampler(j + width * i)
 }
 
-// Lists the slots holding a query of `map`, with the Morton code of the
-// query position (in the scene box) as the sort key.
-__global__ void list_queries_kernel(const float4* __restrict__ slots,
-                                    const float4* __restrict__ srec,
-                                    int64_t n_samples, int q_per_sample, int map,
-                                    float3 lo, float3 inv_ext,
-                                    uint32_t* __restrict__ keys,
-                                    uint32_t* __restrict__ vals,
-                                    unsigned* __restrict__ count) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  // every lane reaches the ballot and the shuffle (no early exit)
-  bool mine = false;
-  float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (t < n_samples * q_per_sample) {
-    const int64_t sidx = t / q_per_sample;
-    const int q = (int)(t % q_per_sample);
-    if (q < __float_as_int(srec[sidx].w)) {
-      mine = __float_as_int(slots[4 * t + 3].w) == map;
-      r0 = slots[4 * t];
+// Lists the slots holding a query of the global map from the front of keys /
+// vals and those of the caustics map from the back (entry n_slots - 1 first),
+// with the Morton code of the query position (in the scene box) as the sort
+// key; count[map] = slots listed. One pass for both maps and one atomic per map
+// and block of 1024 slots: a pass per map with an atomic per warp took 0.56 ms
+// each for 17.8M slots.
+constexpr int kListPer = 4;
+__global__ void __launch_bounds__(256)
+    list_queries_kernel(const float4* __restrict__ slots, const float4* __restrict__ srec,
+                        uint32_t n_used, uint32_t n_slots, uint32_t q_per_sample, float3 lo,
+                        float3 inv_ext, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                        unsigned* __restrict__ count) {
+  __shared__ unsigned warp_n[2][8];
+  __shared__ unsigned block_at[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t t0 = blockIdx.x * (256u * kListPer) + threadIdx.x;
+  int map[kListPer];
+  uint32_t key[kListPer];
+  unsigned at[kListPer];
+  unsigned mine[2] = {0, 0};  // queries of this warp so far
+#pragma unroll
+  for (int r = 0; r < kListPer; ++r) {
+    const uint32_t t = t0 + 256u * r;
+    map[r] = -1;
+    key[r] = 0;
+    if (t < n_used) {
+      const uint32_t sidx = t / q_per_sample;
+      if ((int)(t - sidx * q_per_sample) < __float_as_int(srec[sidx].w)) {
+        map[r] = __float_as_int(slots[4 * (size_t)t + 3].w);
+        const float4 r0 = slots[4 * (size_t)t];
+        auto cell = [](float v, float l, float ie) -> uint32_t {
+          const float c = (v - l) * ie * 1024.f;
+          if (!(c > 0.f)) return 0u;
+          return c >= 1023.f ? 1023u : (uint32_t)c;
+        };
+        key[r] = (spread10(cell(r0.x, lo.x, inv_ext.x)) << 2) |
+                 (spread10(cell(r0.y, lo.y, inv_ext.y)) << 1) |
+                 spread10(cell(r0.z, lo.z, inv_ext.z));
+      }
     }
+    const unsigned b0 = __ballot_sync(kFull, map[r] == kQueryGlobal);
+    const unsigned b1 = __ballot_sync(kFull, map[r] == kQueryCaustics);
+    const unsigned own = map[r] == kQueryGlobal ? b0 : b1;
+    at[r] = (map[r] == kQueryGlobal ? mine[0] : mine[1]) + __popc(own & lt_mask(lane));
+    mine[0] += __popc(b0);
+    mine[1] += __popc(b1);
   }
-  const unsigned bal = __ballot_sync(kFull, mine);
-  unsigned base = 0;
-  const int leader = bal ? __ffs(bal) - 1 : 0;
-  if (bal && (int)lane_id() == leader)
-    base = atomicAdd(count, (unsigned)__popc(bal));
-  base = __shfl_sync(kFull, base, leader);
-  if (!mine) return;
-  const unsigned o = base + __popc(bal & lanemask_lt());
-  auto cell = [](float v, float l, float ie) -> uint32_t {
-    const float c = (v - l) * ie * 1024.f;
-    if (!(c > 0.f)) return 0u;
-    return c >= 1023.f ? 1023u : (uint32_t)c;
-  };
-  keys[o] = (spread10(cell(r0.x, lo.x, inv_ext.x)) << 2) |
-            (spread10(cell(r0.y, lo.y, inv_ext.y)) << 1) |
-            spread10(cell(r0.z, lo.z, inv_ext.z));
-  vals[o] = (uint32_t)t;
+  if (lane < 2) warp_n[lane][warp] = mine[lane];
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned sum = 0;
+    for (int w = 0; w < 8; ++w) {
+      const unsigned n = warp_n[threadIdx.x][w];
+      warp_n[threadIdx.x][w] = sum;
+      sum += n;
+    }
+    block_at[threadIdx.x] = sum ? atomicAdd(count + threadIdx.x, sum) : 0u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kListPer; ++r) {
+    if (map[r] != kQueryGlobal && map[r] != kQueryCaustics) continue;
+    const int m = map[r] == kQueryGlobal ? 0 : 1;
+    const uint32_t i = block_at[m] + warp_n[m][warp] + at[r];
+    const uint32_t o = m == 0 ? i : n_slots - 1u - i;
+    keys[o] = key[r];
+    vals[o] = t0 + 256u * r;
+  }
 }
 
 // Radiance of sample sidx: direct + sum(weight * estimate) over its slots.
@@ -348,10 +378,9 @@ void render_camera(const SceneDev& sc, const RenderArgs& a, cudaStream_t s) {
     camera_kernel<false><<<(n + 127) / 128, 128, 0, s>>>(sc, a);
 }
 
-void render_list_queries(const float4* slots, const float4* srec,
-                         int64_t n_samples, int q_per_sample, int map,
-                         const float* scene_lo, const float* scene_hi,
-                         uint32_t* keys, uint32_t* vals, unsigned* count,
+void render_list_queries(const float4* slots, const float4* srec, int64_t n_samples,
+                         int64_t n_slots, int q_per_sample, const float* scene_lo,
+                         const float* scene_hi, uint32_t* keys, uint32_t* vals, unsigned* count,
                          cudaStream_t s) {
   const int64_t n = n_samples * q_per_sample;
   if (n <= 0) return;
@@ -360,8 +389,10 @@ void render_list_queries(const float4* slots, const float4* srec,
   ie.x = scene_hi[0] > scene_lo[0] ? 1.0f / (scene_hi[0] - scene_lo[0]) : 0.f;
   ie.y = scene_hi[1] > scene_lo[1] ? 1.0f / (scene_hi[1] - scene_lo[1]) : 0.f;
   ie.z = scene_hi[2] > scene_lo[2] ? 1.0f / (scene_hi[2] - scene_lo[2]) : 0.f;
-  list_queries_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-      slots, srec, n_samples, q_per_sample, map, lo, ie, keys, vals, count);
+  constexpr int per = 256 * kListPer;
+  list_queries_kernel<<<(unsigned)((n + per - 1) / per), 256, 0, s>>>(
+      slots, srec, (uint32_t)n, (uint32_t)n_slots, (uint32_t)q_per_sample, lo, ie, keys, vals,
+      count);
 }
 
 void render_resolve(const float4* slots, const float4* srec, const float* res,

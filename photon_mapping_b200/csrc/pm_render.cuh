@@ -47,10 +47,13 @@ void render_path_tracing(const SceneDev& sc, const PathArgs& a, cudaStream_t s);
 
 void render_rng_init(unsigned long long* st, int w, int h, cudaStream_t s);
 void render_camera(const SceneDev& sc, const RenderArgs& a, cudaStream_t s);
-void render_list_queries(const float4* slots, const float4* srec,
-                         int64_t n_samples, int q_per_sample, int map,
-                         const float* scene_lo, const float* scene_hi,
-                         uint32_t* keys, uint32_t* vals, unsigned* count,
+// The slots of the first n_samples samples that hold a query, with Morton keys:
+// those of the global map at the front of keys / vals (n_slots entries), those
+// of the caustics map at the back, last entry first. count: 2 words (zeroed by
+// the caller), slots listed per map. n_slots < 2^31.
+void render_list_queries(const float4* slots, const float4* srec, int64_t n_samples,
+                         int64_t n_slots, int q_per_sample, const float* scene_lo,
+                         const float* scene_hi, uint32_t* keys, uint32_t* vals, unsigned* count,
                          cudaStream_t s);
 // raw != null: write each sample's radiance there instead of accumulating.
 // shadow != null: also add every kept sample to the pixel's FP64 sums
