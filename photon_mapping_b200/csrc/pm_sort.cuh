@@ -2,10 +2,10 @@
 //
 // Per digit pass: rs_hist counts digits per tile, rs_scan_rows scans the
 // digit-major table of tile counts row by row (one block per digit),
-// rs_scatter ranks the tile's pairs by digit in shared memory, equal digits
-// in input order so the sort is stable (deterministic photon indices and
-// Morton order ties), and writes each digit's run of the tile to its place
-// in one contiguous stretch.
+// rs_scatter ranks the tile's pairs by digit, equal digits in input order so
+// the sort is stable (deterministic photon indices and Morton order ties),
+// and writes each digit's run of the tile to its place in one contiguous
+// stretch.
 #pragma once
 
 #include "pm_common.cuh"
@@ -14,22 +14,19 @@ namespace pm {
 
 constexpr int kSortThreads = 256;
 
-// Pairs per tile: the tile's keys and values fit the block's shared memory
-// (36 KB for 64-bit keys, 43 KB for 32-bit keys).
-template <typename K>
-__host__ __device__ constexpr int sort_tile() {
-  return sizeof(K) == 8 ? 2048 : 4096;
-}
+// Pairs per tile, 8 per thread: the tile's keys and values fit the block's
+// shared memory (26 KB for 64-bit keys, 18 KB for 32-bit keys) and a thread's
+// share fits its registers. Tiles of 4096 32-bit pairs leave an SM too few
+// warps: the build of a map takes 267 us instead of 233 us with 20k photons,
+// 758 instead of 729 us with 3M.
+constexpr int kSortTile = 2048;
 
-template <typename K>
-__host__ __device__ constexpr int sort_tiles(int64_t n) {
-  return (int)((n + sort_tile<K>() - 1) / sort_tile<K>());
-}
+constexpr int sort_tiles(int64_t n) { return (int)((n + kSortTile - 1) / kSortTile); }
 
 // Words of the count table for either key type: 256 digits x tiles, then
 // the 256 digit totals.
 constexpr size_t sort_hist_words(int64_t n) {
-  return 256 * (size_t)sort_tiles<unsigned long long>(n) + 256;
+  return 256 * (size_t)sort_tiles(n) + 256;
 }
 
 // Exclusive scan of one value per thread of a kSortThreads block (ws:
@@ -64,9 +61,9 @@ __global__ void __launch_bounds__(kSortThreads)
   const int tid = threadIdx.x;
   h[tid] = 0;
   __syncthreads();
-  const int t0 = blockIdx.x * sort_tile<K>();
+  const int t0 = blockIdx.x * kSortTile;
 #pragma unroll 4
-  for (int r = 0; r < sort_tile<K>() / kSortThreads; ++r) {
+  for (int r = 0; r < kSortTile / kSortThreads; ++r) {
     const int i = t0 + r * kSortThreads + tid;
     if (i < n) atomicAdd(&h[(uint32_t)(kin[i] >> shift) & 255u], 1u);
   }
@@ -109,78 +106,95 @@ static __global__ void __launch_bounds__(kSortThreads)
   if (tid == 0) totals[blockIdx.x] = carry;
 }
 
+// A warp ranks its own consecutive stretch of the tile with counters of its
+// own, so the block meets a fixed few times per tile, not three times per 256
+// pairs. What bounds it is latency: few rounds of dependent shared memory
+// accesses per warp. A map of 1M photons built and used for 65,536 estimates:
+// 520 -> 444 us.
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads)
     rs_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                K* __restrict__ kout, uint32_t* __restrict__ vout, int n,
                int shift, const uint32_t* __restrict__ offs, int ntiles,
                const uint32_t* __restrict__ totals) {
-  constexpr int kTile = sort_tile<K>();
+  constexpr int kTile = kSortTile;
   constexpr int kWarps = kSortThreads / 32;
+  constexpr int kPer = kTile / kSortThreads;  // pairs per thread
   __shared__ K sk[kTile];
   __shared__ uint32_t sv[kTile];
-  __shared__ uint32_t wcnt[kWarps][256];
-  __shared__ uint32_t tstart[256];  // first slot of digit d in the tile
-  __shared__ uint32_t gbase[256];   // output place of that slot
-  __shared__ uint32_t run[256];     // pairs of digit d placed so far
+  __shared__ uint32_t gbase[256];  // output place of digit d's pairs, minus their slot
   __shared__ uint32_t ws[kWarps];
-  const int tid = threadIdx.x, warp = tid >> 5;
+  // pairs of each digit in the earlier rounds of each warp; the keys take its
+  // place once the ranks are known
+  uint32_t(*wcnt)[256] = reinterpret_cast<uint32_t(*)[256]>(sk);
+  static_assert(sizeof(sk) >= sizeof(uint32_t) * kWarps * 256, "counters fit the keys' place");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = blockIdx.x;
   const int t0 = tile * kTile;
   const int cnt = n - t0 < kTile ? n - t0 : kTile;
-  {
-    // digit offset = exclusive scan of the digit totals, plus this tile's
-    // exclusive prefix over the tiles; the tile's own count of digit tid is
-    // the step to the next tile's prefix
-    const uint32_t doff = block_exclusive_scan(totals[tid], ws);
-    const uint32_t pre = offs[tid * ntiles + tile];
-    const uint32_t next = tile + 1 < ntiles ? offs[tid * ntiles + tile + 1] : totals[tid];
-    const uint32_t mine = next - pre;
-    gbase[tid] = doff + pre;
-    tstart[tid] = block_exclusive_scan(mine, ws);
-    run[tid] = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) wcnt[w][tid] = 0;
-    __syncthreads();
+  for (int w = 0; w < kWarps; ++w) wcnt[w][tid] = 0;
+  // digit offset = exclusive scan of the digit totals, plus this tile's
+  // exclusive prefix over the tiles
+  const uint32_t place =
+      block_exclusive_scan(totals[tid], ws) + offs[(size_t)tid * ntiles + tile];
+  // pair r of a thread: warp * 32 * kPer + r * 32 + lane of the tile; equal
+  // digits keep input order (earlier warps, then earlier rounds, then lanes)
+  const int i0 = t0 + warp * (32 * kPer) + lane;
+  K key[kPer];
+  uint32_t val[kPer], slot[kPer];
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int i = i0 + 32 * r;
+    key[r] = i < n ? kin[i] : (K)0;
+    val[r] = i < n ? vin[i] : 0u;
   }
-  // rank: round r holds pairs t0 + r * kSortThreads + tid; equal digits
-  // keep input order (earlier rounds, then earlier warps, then lanes)
-  for (int r = 0; r < kTile / kSortThreads; ++r) {
-    const int i = t0 + r * kSortThreads + tid;
-    const bool ok = i < n;
-    K key = 0;
-    uint32_t val = 0;
-    if (ok) {
-      key = kin[i];
-      val = vin[i];
-    }
-    const uint32_t d = ok ? ((uint32_t)(key >> shift) & 255u) : 0xffffffffu;
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const bool ok = i0 + 32 * r < n;
+    const uint32_t d = ok ? (uint32_t)(key[r] >> shift) & 255u : 256u;
     const unsigned peers = __match_any_sync(kFull, d);
-    const unsigned rank = __popc(peers & lt_mask(tid & 31));
-    if (ok && rank == 0) wcnt[warp][d] = __popc(peers);
-    __syncthreads();
-    if (ok) {
-      uint32_t pos = tstart[d] + run[d] + rank;
-      for (int w = 0; w < warp; ++w) pos += wcnt[w][d];
-      sk[pos] = key;
-      sv[pos] = val;
-    }
-    __syncthreads();
-    uint32_t tot = 0;
+    const uint32_t before = __popc(peers & lt_mask(lane));
+    const uint32_t seen = ok ? wcnt[warp][d] : 0u;
+    __syncwarp();
+    if (ok && before == 0u) wcnt[warp][d] = seen + (uint32_t)__popc(peers);
+    __syncwarp();
+    slot[r] = seen + before;
+  }
+  __syncthreads();
+  {
+    uint32_t sum = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      tot += wcnt[w][tid];
-      wcnt[w][tid] = 0;
+      const uint32_t c = wcnt[w][tid];
+      wcnt[w][tid] = sum;
+      sum += c;
     }
-    run[tid] += tot;
-    __syncthreads();
+    const uint32_t start = block_exclusive_scan(sum, ws);  // first slot of digit tid
+    gbase[tid] = place - start;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) wcnt[w][tid] += start;
   }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    if (i0 + 32 * r < n) slot[r] += wcnt[warp][(uint32_t)(key[r] >> shift) & 255u];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    if (i0 + 32 * r < n) {
+      sk[slot[r]] = key[r];
+      sv[slot[r]] = val[r];
+    }
+  }
+  __syncthreads();
   // write: consecutive slots of one digit go to consecutive places
+#pragma unroll 4
   for (int q = tid; q < cnt; q += kSortThreads) {
-    const K key = sk[q];
-    const uint32_t d = (uint32_t)(key >> shift) & 255u;
-    const uint32_t o = gbase[d] + (uint32_t)q - tstart[d];
-    kout[o] = key;
+    const K k = sk[q];
+    const uint32_t o = gbase[(uint32_t)(k >> shift) & 255u] + (uint32_t)q;
+    kout[o] = k;
     vout[o] = sv[q];
   }
 }
@@ -290,7 +304,7 @@ template <typename K>
 bool radix_sort_pairs(K* ka, uint32_t* va, K* kb, uint32_t* vb, int n,
                       int key_bits, uint32_t* hist, cudaStream_t st) {
   if (n <= 1) return false;
-  const int nt = sort_tiles<K>(n);
+  const int nt = sort_tiles(n);
   bool in_b = false;
   for (int shift = 0; shift < key_bits; shift += 8) {
     const K* kin = in_b ? kb : ka;
