@@ -64,24 +64,24 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
     KnnOut o{};
     o.rgb = (float*)c->r_res.ptr;
     o.stats = c->stats_ptr();
-    if (!slot_adj && use_tiles(c, c->maps[map], nq, map == 0 ? kg : kc, true)) {
+    o.adj_in = slot_adj;
+    o.photon_adj = slot_adj ? photon_adj[map] : nullptr;
+    const int mode = slot_adj ? kModeAdjoint : kModeRadiance;
+    if (use_tiles(c, c->maps[map], nq, map == 0 ? kg : kc, true)) {
       // the sorted keys' places are free: the list of the queries the tiles leave
       uint32_t* left_n = (uint32_t*)((char*)c->r_misc.ptr + 56);
       const TileDefer left{ka, (float*)kb, left_n, false};
       const MapDev m = map_view(c->maps[map]);
       const int k = map == 0 ? kg : kc;
       e = knn_tile_launch(m, a.slots, nq, k, (float)c->map_emitted[map], o.rgb, left,
-                          c->next_counter(), c->num_sms, st, in_b ? vb : va, 4);
+                          c->next_counter(), c->num_sms, st, in_b ? vb : va, 4, o.adj_in, o.photon_adj);
       if (e == cudaSuccess)
-        e = knn_launch(m, a.slots, nq, k, kModeRadiance, (float)c->map_emitted[map], o,
+        e = knn_launch(m, a.slots, nq, k, mode, (float)c->map_emitted[map], o,
                        c->next_counter(), c->num_sms, st, ka, 4, left_n, left.tau);
       if (e != cudaSuccess) return cuda_status(c, e, "render estimates");
       continue;
     }
-    o.adj_in = slot_adj;
-    o.photon_adj = slot_adj ? photon_adj[map] : nullptr;
-    e = knn_launch(map_view(c->maps[map]), a.slots, nq, map == 0 ? kg : kc,
-                   slot_adj ? kModeAdjoint : kModeRadiance, (float)c->map_emitted[map], o,
+    e = knn_launch(map_view(c->maps[map]), a.slots, nq, map == 0 ? kg : kc, mode, (float)c->map_emitted[map], o,
                    c->next_counter(), c->num_sms, st, in_b ? vb : va, 4);
     if (e != cudaSuccess) return cuda_status(c, e, "render estimates");
   }

@@ -234,6 +234,47 @@ __device__ __forceinline__ void tile_bins(const F2 px[4], const F2 py[4], const 
   w1 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
 }
 
+// Adds the adjoints of the kept photons: for query q of the sub-tile and each
+// photon it keeps whose direction its normal (s.sx ..) sees, (s.nx, s.ny, s.nz)[q].
+__device__ __forceinline__ void tile_scatter(const MapDev& m, const TileWarp& s, const uint32_t* sub,
+                                             const uint32_t* words, int rows, int used, int ns,
+                                             int lane, float4* __restrict__ photon_adj) {
+  const int qw = tile_query_words(rows);
+  const uint32_t* mysub = sub + (lane >> 3) * rows;
+#pragma unroll 1
+  for (int t = 0; t < used; t += 4) {
+    uint32_t some = 0;
+    const uint32_t* w = words + 8 * t + lane;
+    for (int q = 0; q < ns; ++q) some |= ~(w[q * qw] + s.below[q]);
+    some &= 0x80808080u;
+    if (!__any_sync(kFull, some != 0u)) continue;
+    const uint4 g = *reinterpret_cast<const uint4*>(mysub + t);
+    const uint32_t gs[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+      if (!(some & (0x80u << (8 * i)))) continue;
+      const uint32_t id = (i < 2 ? (i == 0 ? gs[0] : gs[1]) : (i == 2 ? gs[2] : gs[3])) * kGroup + (lane & 7);
+      const float wx = __ldg(m.thr4 + id).w;
+      const float2 wi = __ldg(m.wi2 + id);
+      const uint32_t to = __float_as_uint(__ldg(m.pos4 + id).w);
+      float3 sum = make_float3(0.f, 0.f, 0.f);
+      bool add = false;
+      for (int q = 0; q < ns; ++q) {
+        const uint32_t keep = ~(w[q * qw] + s.below[q]);
+        // Lambert::evaluate returns 0 when either cosine is < 0
+        if ((keep & (0x80u << (8 * i))) &&
+            !(dot_ref(wx, wi.x, wi.y, s.sx[q], s.sy[q], s.sz[q]) < 0.f)) {
+          sum.x += s.nx[q];
+          sum.y += s.ny[q];
+          sum.z += s.nz[q];
+          add = true;
+        }
+      }
+      if (add) atomicAdd(photon_adj + to, make_float4(sum.x, sum.y, sum.z, 0.f));
+    }
+  }
+}
+
 // Leaves a query to the warp-per-query kernel, with a radius to try.
 __device__ __forceinline__ void leave(const TileDefer& defer, uint32_t query, float tau) {
   const uint32_t o = atomicAdd(defer.count, 1u);
@@ -242,13 +283,16 @@ __device__ __forceinline__ void leave(const TileDefer& defer, uint32_t query, fl
 }
 
 // Queries [q0, q0 + nq) (nq <= 32) in the order of `order`. tau: the squared
-// search radius to try first (in/out).
+// search radius to try first (in/out). A: the adjoint of the estimates, adj_in
+// scattered onto the kept photons in photon_adj, instead of the estimates.
+template <bool A>
 __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, TileWarp& s, int rows,
                                           int lane, const float4* __restrict__ queries,
                                           const uint32_t* __restrict__ order, int stride4,
                                           int64_t q0, int nq, int k, float n_emitted,
                                           float* __restrict__ rgb, const TileDefer& defer,
-                                          float& tau) {
+                                          float& tau, const float* __restrict__ adj_in = nullptr,
+                                          float4* __restrict__ photon_adj = nullptr) {
   uint32_t* const sub = reinterpret_cast<uint32_t*>(&s + 1);
   uint32_t* const words = sub + 4 * rows;  // [query][row / 4][lane]
   uint32_t* const stack = words;           // free during a walk
@@ -264,7 +308,7 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
     pz = r0.z;
   }
   const bool bad = isnan(px) || isnan(py) || isnan(pz);
-  if (lane < nq && bad) rgb[3 * (size_t)rec] = rgb[3 * (size_t)rec + 1] = rgb[3 * (size_t)rec + 2] = 0.f;
+  if (!A && lane < nq && bad) rgb[3 * (size_t)rec] = rgb[3 * (size_t)rec + 1] = rgb[3 * (size_t)rec + 2] = 0.f;
   unsigned todo = __ballot_sync(kFull, lane < nq && !bad);
   float good = tau;      // from the last queries answered
   int span = kTileQ, sq = kSubQ, tries = 0;
@@ -494,6 +538,27 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
       } else if (h == 0) {
         s.sx[qs] = s.sy[qs] = s.sz[qs] = 0.f;
       }
+      uint32_t kth;
+      if constexpr (A) {
+        kth = fit ? s.kth[qs] : 0u;
+        // d estimate / d throughput_i = f(wo, wi_i) / (n_emitted pi maxd2) for
+        // the kept photons (integrator.h:141-150), the warp-per-query kernel's
+        // expression. Lane l adds the queries' parts for its photon of each row,
+        // then adds them to the photon's adjoint at once: a query at a time, the
+        // 50 additions per query to memory bound the pass.
+        float v = fit && h < 3 ? adj_in[3 * (size_t)rq + h] : 0.f;
+        const bool any = (__ballot_sync(kFull, v != 0.f) >> (lane & ~(kLanesQ - 1))) & 0xfu;
+        v = __fdiv_rn(__fmul_rn(v, __fdiv_rn(rho, kPI)),
+                      __fmul_rn(__fmul_rn(n_emitted, kPI), __uint_as_float(kth)));
+        if (!any || cos_o < 0.f) {
+          v = 0.f;
+          if (h == 0) s.below[qs] = 0x80808080u;
+        }
+        // the positions' places
+        if (h < 3) (h == 0 ? s.nx : h == 1 ? s.ny : s.nz)[qs] = v;
+        __syncwarp();
+        tile_scatter(m, s, sub, words, rows, used, ns, lane, photon_adj);
+      } else {
       __syncwarp();
 #pragma unroll 1
       for (int qb = 0; qb < ns; qb += kPassQ) {
@@ -588,9 +653,10 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
         a.w = __fadd_rn(__fadd_rn(a.w, b.w), __fadd_rn(a2.w, b2.w));
         v = __fadd_rn(v, __fadd_rn(__fadd_rn(a.x, a.y), __fadd_rn(a.z, a.w)));
       }
-      const uint32_t kth = fit ? s.kth[qs] : 0u;
+      kth = fit ? s.kth[qs] : 0u;
       if (fit && h < 3)
         rgb[3 * (size_t)rq + h] = radiance_from_sum(v, rho, cos_o, n_emitted, __uint_as_float(kth));
+      }
       if (act && !fit && h == 0)  // the radius up to byte hi holds k photons
         leave(defer, defer.positions ? (uint32_t)(q0 + s.ql[qs]) : rq,
               tf * (float)hi * (1.01f / (float)kBins));
@@ -631,11 +697,13 @@ constexpr int kTileWarps = 4;  // per block
 // 3.13 ms by the warp-per-query kernel. 5 blocks (20 warps) per SM, which the
 // shared memory allows for k = 100, take 96 registers without spills; 4 blocks
 // of 126 registers: 1.250 ms, 6 of 80: spills, 1.40 ms.
+template <bool A>
 __global__ void __launch_bounds__(32 * kTileWarps, 5)
     knn_tile_kernel(MapDev m, const float4* __restrict__ queries,
                     const uint32_t* __restrict__ order, int64_t nq, int stride4, int k,
                     float n_emitted, float* __restrict__ rgb, int rows, int item, TileDefer defer,
-                    unsigned long long* __restrict__ counter) {
+                    unsigned long long* __restrict__ counter, const float* __restrict__ adj_in,
+                    float4* __restrict__ photon_adj) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ TileLevels L;
   const int lane = threadIdx.x & 31;
@@ -645,15 +713,16 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
     for (int i = 0; i < kMaxLevels; ++i) L.oc[i] = make_int2(m.lvl_off[i], m.lvl_cnt[i]);
   }
   __syncthreads();
-  float tau = even_tau(m, m.lvl_off[m.nlevels - 1], k);
+  float tau = even_tau(m, L.oc[m.nlevels - 1].x, k);
   while (true) {
     unsigned long long c0 = 0;
     if (lane == 0) c0 = atomicAdd(counter, 1ull);
     c0 = __shfl_sync(kFull, c0, 0);
     const int64_t q0 = (int64_t)c0 * item;
     if (q0 >= nq) break;
-    tile_item(m, L, s, rows, lane, queries, order, stride4, q0, (int)min((int64_t)item, nq - q0),
-              k, n_emitted, rgb, defer, tau);
+    tile_item<A>(m, L, s, rows, lane, queries, order, stride4, q0,
+                 (int)min((int64_t)item, nq - q0), k, n_emitted, rgb, defer, tau, adj_in,
+                 photon_adj);
     __syncwarp();
   }
 }
@@ -709,8 +778,8 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
       }
       continue;
     }
-    tile_item(wmap[warp], wlev[warp], s, rows, lane, slots, order, 4, q0, nq, k, n_emitted, rgb,
-              defer, tau);
+    tile_item<false>(wmap[warp], wlev[warp], s, rows, lane, slots, order, 4, q0, nq, k,
+                     n_emitted, rgb, defer, tau);
     __syncwarp();
   }
 }
@@ -736,14 +805,16 @@ void query_keys_launch(const MapDev& m, const void* queries, int64_t nq, int str
 cudaError_t knn_tile_launch(const MapDev& m, const void* queries, int64_t nq, int k,
                             float n_emitted, float* rgb, const TileDefer& defer,
                             unsigned long long* counter, int num_sms, cudaStream_t st,
-                            const uint32_t* order, int stride4) {
+                            const uint32_t* order, int stride4, const float* adj_in,
+                            float4* photon_adj) {
+  const auto kern = photon_adj ? knn_tile_kernel<true> : knn_tile_kernel<false>;
   const int rows = tile_rows(k);
   const size_t smem = kTileWarps * tile_bytes(rows);
-  cudaError_t e = cudaFuncSetAttribute(knn_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_tile_kernel, 32 * kTileWarps, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kTileWarps, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   int64_t blocks = (int64_t)num_sms * per_sm;
@@ -759,8 +830,9 @@ cudaError_t knn_tile_launch(const MapDev& m, const void* queries, int64_t nq, in
   if ((e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st)) != cudaSuccess ||
       (e = cudaMemsetAsync(defer.count, 0, sizeof(uint32_t), st)) != cudaSuccess)
     return e;
-  knn_tile_kernel<<<(unsigned)blocks, 32 * kTileWarps, smem, st>>>(
-      m, (const float4*)queries, order, nq, stride4, k, n_emitted, rgb, rows, item, defer, counter);
+  kern<<<(unsigned)blocks, 32 * kTileWarps, smem, st>>>(
+      m, (const float4*)queries, order, nq, stride4, k, n_emitted, rgb, rows, item, defer, counter,
+      adj_in, photon_adj);
   return cudaGetLastError();
 }
 

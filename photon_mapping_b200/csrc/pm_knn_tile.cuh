@@ -40,9 +40,11 @@ void query_keys_launch(const MapDev& m, const void* queries, int64_t nq, int str
 
 constexpr int kTileMinPhotons = 4096;
 constexpr int kTileMaxK = 448;
+// With photon_adj, the adjoint instead (KnnOut::adj_in, photon_adj; rgb unused).
 cudaError_t knn_tile_launch(const MapDev& m, const void* queries, int64_t nq, int k,
                             float n_emitted, float* rgb, const TileDefer& defer,
                             unsigned long long* counter, int num_sms, cudaStream_t st,
-                            const uint32_t* order, int stride4);
+                            const uint32_t* order, int stride4, const float* adj_in = nullptr,
+                            float4* photon_adj = nullptr);
 
 }  // namespace pm
