@@ -170,7 +170,7 @@ extern "C" int pm_diff_forward(pm_ctx* c, const pm_camera* cam, const pm_diff_pa
       (e = cudaMemsetAsync(c->dev_err.ptr, 0, 64, st)))
     return cuda_status(c, e, "render init");
   render_rng_init((unsigned long long*)c->r_rng.ptr, p.width, p.height, st);
-  RenderArgs a = base_args(c, p.width, p.height, q_per_sample, p.final_gathering_depth,
+  RenderArgs a = base_args(c, p.width, p.height, n_samples, q_per_sample, p.final_gathering_depth,
                            p.max_depth, p.n_gather);
   a.cam_pos = v3(cam->position[0], cam->position[1], cam->position[2]);
   a.cam_fwd = v3(cam->forward[0], cam->forward[1], cam->forward[2]);
@@ -282,7 +282,7 @@ extern "C" int pm_diff_backward(pm_ctx* c, const float* grad_rgb, float* grad_al
     if (n > 0 && (e = cudaMemsetAsync(padj[map], 0, (size_t)n * 16, st)))
       return cuda_status(c, e, "photon adjoints");
   }
-  RenderArgs a = base_args(c, d.width, d.height, d.q_per_sample, d.fg_depth, d.max_depth, 1);
+  RenderArgs a = base_args(c, d.width, d.height, n_samples, d.q_per_sample, d.fg_depth, d.max_depth, 1);
   a.batch = d.spp;
   int64_t q_tot[2] = {0, 0};
   if ((s = answer_queries(c, a, n_samples, n_slots, need_caustics, d.k, d.k, q_tot,

@@ -88,8 +88,8 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
   return PM_OK;
 }
 
-RenderArgs base_args(pm_ctx* c, int width, int height, int q_per_sample, int fg_depth,
-                     int max_depth, int n_gather) {
+RenderArgs base_args(pm_ctx* c, int width, int height, int64_t n_samples, int q_per_sample,
+                     int fg_depth, int max_depth, int n_gather) {
   RenderArgs a{};
   a.width = width;
   a.height = height;
@@ -104,6 +104,12 @@ RenderArgs base_args(pm_ctx* c, int width, int height, int q_per_sample, int fg_
   a.sample_rec = (float4*)c->r_srec.ptr;
   a.err = (int*)c->dev_err.ptr;
   a.in_rays = nullptr;
+  if (!c->scene.has_specular && fg_depth > 0 && max_depth > 0) {
+    // 24 bytes per sample in the place of the estimates (12 per slot, at least
+    // 2 slots per sample), which are written when the hits are read no more
+    a.hits = (float4*)c->r_res.ptr;
+    a.hit_rng = (unsigned long long*)(a.hits + n_samples);
+  }
   return a;
 }
 
@@ -166,7 +172,7 @@ extern "C" int pm_render(pm_ctx* c, const pm_camera* cam,
     if ((e = cudaMemsetAsync(shadow, 0, (size_t)npix * 24, st)) != cudaSuccess)
       return cuda_status(c, e, "render init");
   }
-  RenderArgs a = base_args(c, p.width, p.height, q_per_sample, p.final_gathering_depth,
+  RenderArgs a = base_args(c, p.width, p.height, n_samples, q_per_sample, p.final_gathering_depth,
                            p.max_depth, p.n_gather);
   a.cam_pos = v3(cam->position[0], cam->position[1], cam->position[2]);
   a.cam_fwd = v3(cam->forward[0], cam->forward[1], cam->forward[2]);
@@ -285,7 +291,7 @@ extern "C" int pm_integrate(pm_ctx* c, const float* rays, int64_t n,
                            st)) ||
       (e = cudaMemsetAsync(c->dev_err.ptr, 0, 64, st)))
     return cuda_status(c, e, "integrate upload");
-  RenderArgs a = base_args(c, npix, 1, q_per_sample, p.final_gathering_depth, p.max_depth,
+  RenderArgs a = base_args(c, npix, 1, npix, q_per_sample, p.final_gathering_depth, p.max_depth,
                            p.n_gather);
   a.batch = 1;
   a.in_rays = (const float*)c->q_in.ptr;

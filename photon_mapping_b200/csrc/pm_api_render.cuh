@@ -15,7 +15,7 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
                    bool need_caustics, int kg, int kc, int64_t* q_tot,
                    const float* slot_adj, float4* const* photon_adj);
 
-RenderArgs base_args(pm_ctx* c, int width, int height, int q_per_sample, int fg_depth,
+RenderArgs base_args(pm_ctx* c, int width, int height, int64_t n_samples, int q_per_sample, int fg_depth,
                      int max_depth, int n_gather);
 
 // Query slots per sample.

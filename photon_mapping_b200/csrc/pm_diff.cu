@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(128)
       for (int q = 0; q < nq; ++q) {
         const int64_t t = sidx * a.q_per_sample + q;
         const float4 w = a.slots[4 * t + 3];
+        if (__float_as_int(w.w) == kQueryNone) continue;
         rad = rad + v3(w.x, w.y, w.z) *
                         v3(a.res[3 * t], a.res[3 * t + 1], a.res[3 * t + 2]);
       }
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(128)
       for (int q = 0; q < nq; ++q) {
         const int64_t t = sidx * a.q_per_sample + q;
         const float4 w4 = a.slots[4 * t + 3];
+        if (__float_as_int(w4.w) == kQueryNone) continue;
         const V3 w = v3(w4.x, w4.y, w4.z);
         const V3 term = gp * w * v3(a.res[3 * t], a.res[3 * t + 1], a.res[3 * t + 2]);
         const int2 pp = a.slot_pid[t];

@@ -1,6 +1,7 @@
 // Kernels of the differentiable render (see pm_diff.cu).
 #pragma once
 
+#include "pm_render.cuh"
 #include "pm_scene.cuh"
 #include "pm_trace.cuh"
 

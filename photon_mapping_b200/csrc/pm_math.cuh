@@ -78,6 +78,16 @@ struct Rng {
     const uint32_t rot = (uint32_t)(old >> 59u);
     return (xs >> rot) | (xs << ((0u - rot) & 31u));
   }
+  // n draws ahead: the n-fold composition of state -> a state + c by doubling
+  // (Brown, "Random number generation with arbitrary strides", 1994).
+  __device__ __forceinline__ void skip(int n) {
+    unsigned long long a = 6364136223846793005ull, c = 1ull;
+    for (; n > 0; n >>= 1) {
+      if (n & 1) state = state * a + c;
+      c = (a + 1ull) * c;
+      a = a * a;
+    }
+  }
   __device__ __forceinline__ float next1d() {
     return (float)next_u32() * (1.0f / 4294967295.0f);
   }

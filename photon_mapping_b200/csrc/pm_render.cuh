@@ -5,7 +5,7 @@
 
 namespace pm {
 
-enum { kQueryGlobal = 0, kQueryCaustics = 1 };
+enum { kQueryNone = -1, kQueryGlobal = 0, kQueryCaustics = 1 };  // map of a query slot
 
 struct RenderArgs {
   V3 cam_pos, cam_fwd, cam_right, cam_up;
@@ -21,6 +21,11 @@ struct RenderArgs {
   float4* slots;       // 4 float4 per query slot
   float4* sample_rec;  // per sample {direct radiance, query count bits}
   const float* in_rays;  // null: camera rays; else 6 floats per pixel slot
+  // Per sample, the first hit {t, u, v, face bits or -1} and the sampler's state
+  // before the sample: not null when all materials are Lambert and fg_depth and
+  // max_depth are positive.
+  float4* hits;
+  unsigned long long* hit_rng;
   int* err;            // bit 1: slots exhausted, bit 2: path stack full
   // Differentiable render (null otherwise): what the adjoint pass needs to
   // split each sample's radiance by albedo parameter.
