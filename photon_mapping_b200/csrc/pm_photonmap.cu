@@ -47,17 +47,28 @@ size_t map_build_scratch_bytes(int64_t n) {
 }
 
 
-__global__ void bbox_kernel(const float* __restrict__ aos, int n,
+constexpr int kBoxThreads = 256;
+__global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const float* __restrict__ aos, int n,
                             uint32_t* __restrict__ bb) {
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
   float hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x) {
+  // four records in flight per thread
+  const int step = gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * (int64_t)step) {
+    float v[4][3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float v = aos[9 * (size_t)i + 3 + a];
-      lo[a] = fminf(lo[a], v);  // fminf ignores NaN
-      hi[a] = fmaxf(hi[a], v);
+    for (int r = 0; r < 4; ++r) {
+      const int64_t j = min(i + (int64_t)r * step, (int64_t)n - 1);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) v[r][a] = __ldg(aos + 9 * j + 3 + a);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        lo[a] = fminf(lo[a], v[r][a]);  // fminf ignores NaN
+        hi[a] = fmaxf(hi[a], v[r][a]);
+      }
     }
   }
 #pragma unroll
@@ -68,12 +79,23 @@ __global__ void bbox_kernel(const float* __restrict__ aos, int n,
       hi[a] = fmaxf(hi[a], __shfl_xor_sync(kFull, hi[a], o));
     }
   }
+  // one atomic per block and bound: those to one address are serial (one per
+  // warp, 3.26M photons: 53 us, 20 us this way)
+  __shared__ float part[6][kBoxThreads / 32];
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      atomicMin(&bb[a], ordered_bits(lo[a]));
-      atomicMax(&bb[3 + a], ordered_bits(hi[a]));
+      part[a][threadIdx.x >> 5] = lo[a];
+      part[3 + a][threadIdx.x >> 5] = hi[a];
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const int c = threadIdx.x;
+    float v = part[c][0];
+    for (int w = 1; w < kBoxThreads / 32; ++w) v = c < 3 ? fminf(v, part[c][w]) : fmaxf(v, part[c][w]);
+    if (c < 3) atomicMin(&bb[c], ordered_bits(v));
+    else atomicMax(&bb[c], ordered_bits(v));
   }
 }
 
@@ -181,7 +203,7 @@ void map_build_launch(const float* aos, int n, float4* pos4, float4* thr4,
   cudaMemsetAsync(bb + 3, 0x00, 3 * sizeof(uint32_t), st);
   const int tb = 256;
   const int gb = (n + tb - 1) / tb;
-  bbox_kernel<<<min(gb, 1184), tb, 0, st>>>(aos, n, bb);
+  bbox_kernel<<<min((n + 4 * kBoxThreads - 1) / (4 * kBoxThreads), 592), kBoxThreads, 0, st>>>(aos, n, bb);
   morton_kernel<<<gb, tb, 0, st>>>(aos, n, bb, ka, va);
   const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, n, 30, hist, st);
   const int places = (int)map_places(n);
