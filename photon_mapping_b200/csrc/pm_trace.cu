@@ -225,15 +225,21 @@ __device__ __forceinline__ bool photon_ray(const TraceArgs& a, const PhotonPath&
 //   * lanes with a ray visit nodes until `shade` lanes have their closest hit;
 //     those shade and start their next ray while the others keep their place in
 //     the tree;
-//   * leaves met are tested together, once `test` lanes wait for one.
+//   * leaves met wait in a queue, and the lanes that can go on in the tree do; a
+//     triangle is tested when as many lanes have one waiting as could visit a
+//     node. Waiting longer costs more visits than it saves tests: a test is what
+//     shortens the ray (1M photons: box 0.97, caustics scene 3.58 and 7.55 ms
+//     when lanes stop at a leaf until 8 do; with a queue tested by 8 lanes 0.98,
+//     3.72, 7.64, by 20 lanes 1.04, 5.21, 10.5; this rule 0.91, 3.33, 7.40).
 // The photons traced, and what they store, do not depend on which thread traces
 // them or in which order.
 // scene(src) and args(src) give the scene and trace arguments of source src
 // (a scene of a batch, or the kernel's only one); first(g, src) maps the
 // work index g to (source, photon index).
-template <int MODE, int STACK, class Scene, class Args, class First>
+// queue: the thread's first place of kLeafQueue * BLOCK in shared memory.
+template <int MODE, int STACK, int BLOCK, class Scene, class Args, class First>
 __device__ __forceinline__ void trace_persistent(unsigned long long* next, long long total,
-                                                 int shade, int test, ReplaySmem* rs,
+                                                 int shade, ReplaySmem* rs, int* queue,
                                                  Scene&& scene, Args&& args, First&& first) {
   const int lane = (int)(threadIdx.x & 31);
   PhotonPath p;
@@ -281,7 +287,7 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
       const TraceArgs& a = args(src);
       photon_leave<MODE>(sc, a, p, v, light, rs);
       if (photon_ray<MODE>(a, p)) {
-        w.start(sc, p.org, p.dir, kRayEps, __int_as_float(0x7f7fffff));
+        w.start(sc, p.org, p.dir, kRayEps, __int_as_float(0x7f7fffff), queue);
         ++nrays;
         state = kWalk;
       } else {
@@ -297,11 +303,12 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
       if (state == kWalk && w.over()) state = kHit;
       const unsigned walking = __ballot_sync(kFull, state == kWalk);
       if (walking == 0 || live - __popc(walking) >= enough) break;
-      const unsigned leaf = __ballot_sync(kFull, state == kWalk && w.at_leaf());
-      if (__popc(leaf) >= test || leaf == walking) {
-        if (state == kWalk && w.at_leaf()) w.test(p.org, p.dir);
+      const unsigned leaf = __ballot_sync(kFull, state == kWalk && w.waiting > 0);
+      const unsigned inner = __ballot_sync(kFull, state == kWalk && w.can_visit());
+      if (__popc(leaf) >= __popc(inner)) {  // a walking lane is in one of them: never both empty
+        if (state == kWalk && w.waiting > 0) w.test<BLOCK>(p.org, p.dir, queue);
       } else {
-        if (state == kWalk && !w.at_leaf()) w.visit(stack, scene(src).err);
+        if (state == kWalk && w.can_visit()) w.visit<BLOCK>(stack, queue, scene(src).err);
       }
     }
   }
@@ -312,9 +319,13 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
   }
 }
 
+constexpr int kTraceBlock = 128;       // threads; ReplaySmem holds as many counters
+constexpr int kBatchTraceBlock = 256;  // and of a batch
+
 template <int MODE>
-__global__ void __launch_bounds__(128, 6)
-    trace_kernel(SceneDev sc, TraceArgs a, int shade, int test) {
+__global__ void __launch_bounds__(kTraceBlock, 6)
+    trace_kernel(SceneDev sc, TraceArgs a, int shade) {
+  __shared__ int queue[kLeafQueue * kTraceBlock];
   auto scene = [&](int) -> const SceneDev& { return sc; };
   auto args = [&](int) -> const TraceArgs& { return a; };
   auto first = [](long long g, int& src) {
@@ -325,21 +336,24 @@ __global__ void __launch_bounds__(128, 6)
     __shared__ ReplaySmem rs;
     for (int t = threadIdx.x; t < 3 * a.n_params; t += blockDim.x) rs.g[t] = 0.f;
     __syncthreads();
-    trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, shade, test, &rs, scene, args, first);
+    trace_persistent<MODE, kBvhStack, kTraceBlock>(a.next, a.n_emit, shade, &rs,
+                                                   &queue[threadIdx.x], scene, args, first);
     __syncthreads();
     for (int t = threadIdx.x; t < 3 * a.n_params; t += blockDim.x)
       if (rs.g[t] != 0.f) atomicAdd(a.grad + t, (double)rs.g[t]);
     return;
   }
-  trace_persistent<MODE, kBvhStack>(a.next, a.n_emit, shade, test, nullptr, scene, args, first);
+  trace_persistent<MODE, kBvhStack, kTraceBlock>(a.next, a.n_emit, shade, nullptr,
+                                                 &queue[threadIdx.x], scene, args, first);
 }
 
 // Every emitted photon of every scene of a batch: the global map rule, each
 // scene appending to its own region. Persistent: the photon index runs over
 // all scenes' photons, the scene found by binary search.
 template <int STACK>
-__global__ void __launch_bounds__(256, 3)
-    batch_trace_kernel(BatchTables t, int64_t total, int shade, int test) {
+__global__ void __launch_bounds__(kBatchTraceBlock, 3)
+    batch_trace_kernel(BatchTables t, int64_t total, int shade) {
+  __shared__ int queue[kLeafQueue * kBatchTraceBlock];
   __shared__ int64_t off[kMaxBatchScenes + 1];
   batch_load_offsets(off, t.emit_off, t.n_scenes);
   __syncthreads();
@@ -349,7 +363,8 @@ __global__ void __launch_bounds__(256, 3)
     src = batch_find(off, t.n_scenes, g);
     return (int)(g - off[src]);
   };
-  trace_persistent<kTracePlain, STACK>(t.next_photon, total, shade, test, nullptr, scene, args, first);
+  trace_persistent<kTracePlain, STACK, kBatchTraceBlock>(t.next_photon, total, shade, nullptr,
+                                                         &queue[threadIdx.x], scene, args, first);
 }
 
 static int sm_count() {
@@ -359,16 +374,13 @@ static int sm_count() {
   return sms;
 }
 
-// Lanes with a hit that end a walk, and lanes at a leaf that start a test
-// (trace_persistent). With several paths per resident lane (24 warps per SM)
-// warps stay full and 20 of 32 is the best (1M photons: caustics scene 4.76 ->
-// 3.56 ms, Cornell box 1.04 -> 0.97 ms; 16 and 24 within 6 %); with fewer, the
-// time is that of the longest paths, which waiting lanes would stretch (100k
-// photons in the box: 0.27 ms, 0.31 ms with 20).
-static void trace_pace(int64_t paths, int* shade, int* test) {
-  const bool full = paths >= 4 * (int64_t)sm_count() * 24 * 32;
-  *shade = full ? 20 : 32;
-  *test = full ? 8 : 1;
+// Lanes with a hit that end a walk (trace_persistent). With several paths per
+// resident lane (24 warps per SM) warps stay full and 20 of 32 is the best (1M
+// photons, caustics scene: 16 and 24 within 2 %); with fewer, the time is that of
+// the longest paths, which waiting lanes would stretch (100k photons in the box:
+// 0.27 ms, 0.31 ms with 20).
+static int trace_pace(int64_t paths) {
+  return paths >= 4 * (int64_t)sm_count() * 24 * 32 ? 20 : 32;
 }
 
 void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int stack,
@@ -378,31 +390,29 @@ void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int
   const long long cap = (long long)sm_count() * (2048 / block);
   const unsigned gb = (unsigned)std::min<long long>(cap, (total_emit + block - 1) / block);
   cudaMemsetAsync(t.next_photon, 0, sizeof(unsigned long long), st);
-  int shade, test;
-  trace_pace(total_emit, &shade, &test);
+  const int shade = trace_pace(total_emit);
   if (stack <= 16)
-    batch_trace_kernel<16><<<gb, block, 0, st>>>(t, total_emit, shade, test);
+    batch_trace_kernel<16><<<gb, block, 0, st>>>(t, total_emit, shade);
   else if (stack <= 32)
-    batch_trace_kernel<32><<<gb, block, 0, st>>>(t, total_emit, shade, test);
+    batch_trace_kernel<32><<<gb, block, 0, st>>>(t, total_emit, shade);
   else
-    batch_trace_kernel<64><<<gb, block, 0, st>>>(t, total_emit, shade, test);
+    batch_trace_kernel<64><<<gb, block, 0, st>>>(t, total_emit, shade);
 }
 
 void trace_launch(const SceneDev& sc, const TraceArgs& a, cudaStream_t st) {
   if (a.n_emit <= 0) return;
-  const int tb = 128;  // ReplaySmem holds 128 threads' counters
+  const int tb = kTraceBlock;
   // persistent: as many blocks as fit at once (2048 threads per SM)
   const long long cap = (long long)sm_count() * (2048 / tb);
   const int gb = (int)std::min<long long>(cap, (a.n_emit + tb - 1) / tb);
   cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), st);
-  int shade, test;
-  trace_pace(a.n_emit, &shade, &test);
+  const int shade = trace_pace(a.n_emit);
   if (a.adj)
-    trace_kernel<kTraceReplay><<<gb, tb, 0, st>>>(sc, a, shade, test);
+    trace_kernel<kTraceReplay><<<gb, tb, 0, st>>>(sc, a, shade);
   else if (a.dmat)
-    trace_kernel<kTraceFrozen><<<gb, tb, 0, st>>>(sc, a, shade, test);
+    trace_kernel<kTraceFrozen><<<gb, tb, 0, st>>>(sc, a, shade);
   else
-    trace_kernel<kTracePlain><<<gb, tb, 0, st>>>(sc, a, shade, test);
+    trace_kernel<kTracePlain><<<gb, tb, 0, st>>>(sc, a, shade);
 }
 
 // out[first[p] + j] = the record with key p << 8 | j. A warp moves 32 consecutive
