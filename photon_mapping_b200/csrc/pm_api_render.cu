@@ -104,7 +104,8 @@ RenderArgs base_args(pm_ctx* c, int width, int height, int64_t n_samples, int q_
   a.sample_rec = (float4*)c->r_srec.ptr;
   a.err = (int*)c->dev_err.ptr;
   a.in_rays = nullptr;
-  if (!c->scene.has_specular && fg_depth > 0 && max_depth > 0) {
+  a.lambert = !c->scene.has_specular && max_depth > 0;
+  if (a.lambert && fg_depth > 0) {
     // 24 bytes per sample in the place of the estimates (12 per slot, at least
     // 2 slots per sample), which are written when the hits are read no more
     a.hits = (float4*)c->r_res.ptr;

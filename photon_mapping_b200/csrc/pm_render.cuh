@@ -21,9 +21,9 @@ struct RenderArgs {
   float4* slots;       // 4 float4 per query slot
   float4* sample_rec;  // per sample {direct radiance, query count bits}
   const float* in_rays;  // null: camera rays; else 6 floats per pixel slot
+  bool lambert;  // all materials are Lambert, and max_depth is positive
   // Per sample, the first hit {t, u, v, face bits or -1} and the sampler's state
-  // before the sample: not null when all materials are Lambert and fg_depth and
-  // max_depth are positive.
+  // before the sample: not null when also fg_depth is positive.
   float4* hits;
   unsigned long long* hit_rng;
   int* err;            // bit 1: slots exhausted, bit 2: path stack full

@@ -32,28 +32,30 @@ def pair(ctx, n_photons, k, fg, max_depth, seed):
         yield pmi
 
 
+@pytest.mark.parametrize("fg", (0, 1))
 @pytest.mark.parametrize("w,h,spp,n_gather,batch,max_depth,back",
                          [(33, 17, 5, 1, 0, 100, 0.0), (16, 16, 3, 7, 2, 100, 1.5), (1, 1, 4, 64, 1, 1, 0.0),
                           (40, 9, 1, 2, 0, 2, 4.0)])
-def test_split_pass_is_the_path_pass(ctx, w, h, spp, n_gather, batch, max_depth, back):
+def test_split_pass_is_the_path_pass(ctx, w, h, spp, n_gather, batch, max_depth, back, fg):
     pos = np.asarray(S.CAMERA["position"], np.float32) - back * np.asarray(S.CAMERA["forward"],
                                                                            np.float32)
     cam = Camera(pos, S.CAMERA["forward"], S.CAMERA["fov"])
     got = [pmi.render(cam, w, h, spp, n_gather=n_gather, spp_batch=batch)
-           for pmi in pair(ctx, 5000, 20, 1, max_depth, 3)]
+           for pmi in pair(ctx, 5000, 20, fg, max_depth, 3)]
     assert np.isfinite(got[0][0]).all()
     np.testing.assert_array_equal(got[0][0], got[1][0])
     for key in ("rays", "queries_global", "queries_caustics", "dropped_nan", "dropped_negative"):
         assert got[0][1][key] == got[1][1][key], key
 
 
-def test_integrated_rays_and_their_samplers(ctx):
+@pytest.mark.parametrize("fg", (0, 1))
+def test_integrated_rays_and_their_samplers(ctx, fg):
     rng = np.random.default_rng(1)
     n = 129
     o = rng.uniform(0.1, 0.9, (n, 3)).astype(np.float32)
     d = rng.normal(size=(n, 3)).astype(np.float32)
     d /= np.linalg.norm(d, axis=1, keepdims=True)
     st = rng.integers(0, 1 << 62, n).astype(np.uint64)
-    got = [pmi.integrate_batch(o, d, st, n_gather=3) for pmi in pair(ctx, 5000, 20, 1, 100, 3)]
+    got = [pmi.integrate_batch(o, d, st, n_gather=3) for pmi in pair(ctx, 5000, 20, fg, 100, 3)]
     np.testing.assert_array_equal(got[0][0], got[1][0])
     np.testing.assert_array_equal(got[0][1], got[1][1])
