@@ -60,6 +60,12 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
     // the caustics map's list lies at the end
     const size_t at = map == 0 ? 0 : (size_t)n_slots - nq;
     uint32_t *ka = keys_a + at, *kb = keys_b + at, *va = vals_a + at, *vb = vals_b + at;
+    if (c->maps[map].n == 0 && !c->stats_on) {
+      // no photon: estimates of 0 and nothing for the adjoint (the caustics map of
+      // a scene of Lambert surfaces: sort and search of 1M queries took 0.35 ms)
+      if (!slot_adj) render_zero_estimates(va, nq, (float*)c->r_res.ptr, st);
+      continue;
+    }
     const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, (int)nq, 30, hist, st);
     KnnOut o{};
     o.rgb = (float*)c->r_res.ptr;

@@ -28,7 +28,7 @@ struct DiffAdjointArgs {
                            // the emission (d loss / d log parameter)
 };
 
-// One thread per pixel: the reverse of resolve + finish. Samples that the
+// One thread per sample: the reverse of resolve + finish. Samples that the
 // forward pass dropped (NaN or negative radiance) get no adjoint.
 void diff_adjoint_samples_launch(const DiffAdjointArgs& a, cudaStream_t st);
 

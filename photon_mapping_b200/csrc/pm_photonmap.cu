@@ -225,8 +225,9 @@ void map_build_launch(const float* aos, int n, float4* pos4, float4* thr4,
 //   1. bound: an upper bound tau of the k-th distance. From the previous
 //      query of the chunk by the triangle inequality when it is close
 //      ((r_prev + delta)^2, inflated for rounding; first tried at the
-//      smaller (1.06 r_prev)^2, kept when it holds k photons), else from
-//      the photons Morton-adjacent to the group nearest the query.
+//      smaller (1.06 r_prev)^2, kept when it holds k photons), else a guess
+//      grown until it holds k photons, at last from the photons
+//      Morton-adjacent to the group nearest the query.
 //   2. collect: depth-first walk of the 32-ary box tree; the passing
 //      8-photon groups of a node are scanned packed, 4 groups per round,
 //      every photon with dist2 <= tau appended to the warp's buffer. A

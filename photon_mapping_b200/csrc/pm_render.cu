@@ -442,6 +442,18 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+__global__ void zero_estimates_kernel(const uint32_t* __restrict__ vals, unsigned n,
+                                      float* __restrict__ res) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const size_t t = vals[i];
+  res[3 * t] = res[3 * t + 1] = res[3 * t + 2] = 0.f;
+}
+
+void render_zero_estimates(const uint32_t* vals, unsigned n, float* res, cudaStream_t s) {
+  if (n > 0) zero_estimates_kernel<<<(n + 255) / 256, 256, 0, s>>>(vals, n, res);
+}
+
 // Radiance of sample sidx: direct + sum(weight * estimate) over its slots.
 __device__ __forceinline__ V3 sample_radiance(const float4* __restrict__ slots,
                                               const float4* __restrict__ srec,

@@ -60,6 +60,8 @@ void render_list_queries(const float4* slots, const float4* srec, int64_t n_samp
                          int64_t n_slots, int q_per_sample, const float* scene_lo,
                          const float* scene_hi, uint32_t* keys, uint32_t* vals, unsigned* count,
                          cudaStream_t s);
+// The estimates of the listed slots in a map without photons.
+void render_zero_estimates(const uint32_t* vals, unsigned n, float* res, cudaStream_t s);
 // raw != null: write each sample's radiance there instead of accumulating.
 // shadow != null: also add every kept sample to the pixel's FP64 sums
 // (3 doubles per pixel).

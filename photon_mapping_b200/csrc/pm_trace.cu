@@ -1,5 +1,5 @@
 // Photon emission and tracing on the device (PhotonMapping::build,
-// integrator.h:393-563), one thread per emitted photon.
+// integrator.h:393-563), a lane per photon path in persistent warps.
 //
 // Random numbers: photon i draws from its own UniformSampler-style PCG32
 // stream whose state starts at photon_stream_state(seed, i); the draws

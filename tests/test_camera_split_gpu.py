@@ -59,3 +59,23 @@ def test_integrated_rays_and_their_samplers(ctx, fg):
     got = [pmi.integrate_batch(o, d, st, n_gather=3) for pmi in pair(ctx, 5000, 20, fg, 100, 3)]
     np.testing.assert_array_equal(got[0][0], got[1][0])
     np.testing.assert_array_equal(got[0][1], got[1][1])
+
+
+def test_estimates_in_an_empty_map_are_zero(ctx):
+    """Lambert scenes store no caustics photons: their caustics estimates are
+    zeros written without a search, which statistics switch on again."""
+    cam = Camera(S.CAMERA["position"], S.CAMERA["forward"], S.CAMERA["fov"])
+    scene = S.Scene(ctx)
+    scene.setMesh(S.cornell_box(2))
+    scene.build()
+    pmi = PhotonMapping(5000, 20, 1.0, 20, 1, 100, ctx=ctx)
+    pmi.build(scene, seed=3)
+    img, st = pmi.render(cam, 31, 17, 2)
+    assert st["queries_caustics"] > 0
+    ctx.set_stats(True)
+    try:
+        want, wst = pmi.render(cam, 31, 17, 2)
+    finally:
+        ctx.set_stats(False)
+    np.testing.assert_array_equal(img, want)
+    assert st["queries_caustics"] == wst["queries_caustics"]
