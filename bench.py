@@ -43,6 +43,9 @@ SPP = 4                     # the query frame: primary hits of 512x512x4 spp
 # algorithmic bytes per query: k photons x 36 B (position, throughput, wi),
 # the 48-B radiance query record in (position, wo, shading normal, albedo)
 # and the 12-B RGB out
+# launches of one estimate call of this size: the queries' keys, a sort of 3 digits with
+# 3 kernels each, the tile kernel, the warp-per-query kernel for what it leaves
+LAUNCHES_PER_STEP = 12
 BYTES_PER_QUERY = 36 * K_NEAREST + 48 + 12
 METRIC = "kNN radiance queries/s at 1M photons k=100"
 CPU_SAMPLE_QUERIES = 40000
@@ -194,9 +197,9 @@ def measured_peak_hbm() -> tuple[float, str]:
 
 
 def ncu_traffic() -> float | None:
-    """DRAM bytes per launch of the kNN radiance kernel from the committed
-    ncu summary (profiles/knn_radiance_traffic.json), scaled to this
-    workload's query count when the capture ran a smaller case."""
+    """DRAM bytes of one estimate call (its LAUNCHES_PER_STEP launches) from the
+    committed ncu summary (profiles/knn_radiance_traffic.json), of a call with
+    3 % fewer queries."""
     p = ROOT / "profiles" / "knn_radiance_traffic.json"
     if not p.exists():
         return None
@@ -702,7 +705,7 @@ def run_ours(args) -> None:
         "e2e": {"value": e2e_value, "unit": "queries/s",
                 "h2d_bytes_per_step": int(queries.nbytes),
                 "d2h_bytes_per_step": int(nq * 3 * 4)},
-        "gpu_launches": args.steps,
+        "gpu_launches": args.steps * LAUNCHES_PER_STEP,
         "parity": parity,
         "knn_per_query": per_q,
         "knn_uniform_cube": uniform,
