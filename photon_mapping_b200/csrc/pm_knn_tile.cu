@@ -795,6 +795,16 @@ int tile_rows(int k) {
 }
 static_assert(tile_query_words(16) >= 3 * 36, "place of the sums");
 
+// Lets a tile kernel use the shared memory of the largest k, whatever k it is
+// launched for: the limit belongs to the function, so one set for a single k
+// would be another context's or batch's limit too, which may launch for a
+// larger k in between.
+template <class F>
+static cudaError_t allow_tile_smem(F kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(kTileWarps * tile_bytes(tile_rows(kTileMaxK))));
+}
+
 void query_keys_launch(const MapDev& m, const void* queries, int64_t nq, int stride4,
                        uint32_t* keys, uint32_t* vals, cudaStream_t st) {
   if (nq <= 0) return;
@@ -810,8 +820,7 @@ cudaError_t knn_tile_launch(const MapDev& m, const void* queries, int64_t nq, in
   const auto kern = photon_adj ? knn_tile_kernel<true> : knn_tile_kernel<false>;
   const int rows = tile_rows(k);
   const size_t smem = kTileWarps * tile_bytes(rows);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  cudaError_t e = allow_tile_smem(kern);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kTileWarps, smem);
@@ -844,8 +853,7 @@ int batch_tile_item(int64_t nq, int num_sms) {
 
 cudaError_t batch_tile_prepare(int max_k, int* blocks_per_sm) {
   const size_t smem = kTileWarps * tile_bytes(tile_rows(max_k));
-  cudaError_t e = cudaFuncSetAttribute(
-      knn_tile_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_tile_smem(knn_tile_batch_kernel);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_tile_batch_kernel,

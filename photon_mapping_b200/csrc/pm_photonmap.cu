@@ -1234,7 +1234,9 @@ cudaError_t batch_knn_prepare(int warps, int buffer, int* blocks_per_sm) {
   auto kern = buffer <= 512 ? knn_batch_kernel<512> : knn_batch_kernel<2048>;
   const size_t smem =
       (size_t)warps * (buffer <= 512 ? sizeof(WarpBuf<512>) : sizeof(WarpBuf<2048>));
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is the function's, shared by all batches: always that of 8 warps
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(smem / warps * 8));
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
