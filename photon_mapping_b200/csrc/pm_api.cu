@@ -152,7 +152,10 @@ int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq,
   StreamScratch* sc = nullptr;
   int s = take_scratch(c, words * 4, st, &sc);
   if (s != PM_OK) return s;
-  uint32_t* ka = (uint32_t*)sc->buf.ptr;
+  // the work counter, for one launch after the other: like the rest of the
+  // buffer it is nobody else's until `done`, however many calls are in flight
+  unsigned long long* counter = (unsigned long long*)sc->buf.ptr;
+  uint32_t* ka = (uint32_t*)sc->buf.ptr + 16;
   uint32_t* kb = ka + nq;
   uint32_t* va = kb + nq;
   uint32_t* vb = va + nq;
@@ -162,13 +165,13 @@ int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq,
   const bool in_b = radix_sort_pairs<uint32_t>(ka, va, kb, vb, (int)nq, kQueryKeyBits, hist, st);
   // the keys' places are free again: the list of the queries left
   const TileDefer left{ka, (float*)kb, hist, false};
-  cudaError_t e = knn_tile_launch(m, d_q, nq, k, n_emitted, d_rgb, left, c->next_counter(),
-                                  c->num_sms, st, in_b ? vb : va, 3);
+  cudaError_t e = knn_tile_launch(m, d_q, nq, k, n_emitted, d_rgb, left, counter, c->num_sms,
+                                  st, in_b ? vb : va, 3);
   if (e == cudaSuccess) {
     KnnOut o{};
     o.rgb = d_rgb;
-    e = knn_launch(m, d_q, nq, k, kModeRadiance, n_emitted, o, c->next_counter(), c->num_sms, st,
-                   ka, 3, hist, left.tau);
+    e = knn_launch(m, d_q, nq, k, kModeRadiance, n_emitted, o, counter, c->num_sms, st, ka, 3,
+                   hist, left.tau);
   }
   const cudaError_t e2 = cudaEventRecord(sc->done, st);
   return cuda_status(c, e != cudaSuccess ? e : e2, "radiance launch");

@@ -79,11 +79,12 @@ int answer_queries(pm_ctx* c, const RenderArgs& a, int64_t ns, int64_t n_slots,
       const TileDefer left{ka, (float*)kb, left_n, false};
       const MapDev m = map_view(c->maps[map]);
       const int k = map == 0 ? kg : kc;
-      e = knn_tile_launch(m, a.slots, nq, k, (float)c->map_emitted[map], o.rgb, left,
-                          c->next_counter(), c->num_sms, st, in_b ? vb : va, 4, o.adj_in, o.photon_adj);
+      unsigned long long* counter = c->next_counter();  // for one launch after the other
+      e = knn_tile_launch(m, a.slots, nq, k, (float)c->map_emitted[map], o.rgb, left, counter,
+                          c->num_sms, st, in_b ? vb : va, 4, o.adj_in, o.photon_adj);
       if (e == cudaSuccess)
-        e = knn_launch(m, a.slots, nq, k, mode, (float)c->map_emitted[map], o,
-                       c->next_counter(), c->num_sms, st, ka, 4, left_n, left.tau);
+        e = knn_launch(m, a.slots, nq, k, mode, (float)c->map_emitted[map], o, counter, c->num_sms,
+                       st, ka, 4, left_n, left.tau);
       if (e != cudaSuccess) return cuda_status(c, e, "render estimates");
       continue;
     }

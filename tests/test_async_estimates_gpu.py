@@ -1,0 +1,59 @@
+"""pm_photonmap_radiance_device as an asynchronous call: many in flight, on one stream
+and on several, beside a capture, and without memory for its query buffers."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from photon_mapping_b200 import Context, PhotonMap
+from photon_mapping_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+N, K = 100_000, 50
+MIN_QUERIES = 5_000_000 // (K + 50)  # fewest that tiles answer
+
+
+@pytest.fixture
+def own():
+    """A context of its own: no query buffers yet."""
+    with Context(0) as c:
+        pm = PhotonMap(c)
+        pm.setPhotons(W.wall_photons(N, 1))
+        pm.build()
+        yield c
+
+
+def call(ctx, q, out, stream):
+    ctx.check(ctx.lib.pm_photonmap_radiance_device(
+        ctx.handle, 0, q.data_ptr(), q.shape[0], K, N, out.data_ptr(), stream.cuda_stream),
+        "pm_photonmap_radiance_device")
+
+
+def alone(ctx, q):
+    import torch
+    o = torch.empty((q.shape[0], 3), device="cuda")
+    call(ctx, q, o, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    return o
+
+
+def test_more_calls_in_flight_than_the_context_has_counters(own):
+    import torch
+    long_q = torch.from_numpy(W.wall_queries(8 * MIN_QUERIES, 2)).cuda()
+    short = [torch.from_numpy(W.wall_queries(MIN_QUERIES + 999 * i, 3 + i)).cuda()
+             for i in range(6)]
+    long_want, want = alone(own, long_q), [alone(own, q) for q in short]
+    first, others = torch.cuda.Stream(), [torch.cuda.Stream() for _ in short]
+    long_got = [torch.zeros_like(long_want) for _ in range(80)]
+    got = [[torch.zeros_like(w) for w in want] for _ in range(12)]
+    torch.cuda.synchronize()
+    for o in long_got:
+        call(own, long_q, o, first)
+    for row in got:
+        for q, o, s in zip(short, row, others):
+            call(own, q, o, s)
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, long_want) for o in long_got)
+    for row in got:
+        assert all(torch.equal(o, w) for o, w in zip(row, want))
