@@ -424,7 +424,8 @@ typedef struct pm_batch_scene {
 /* Launch shapes of the batched kernels (pm_batch_autotune picks them). */
 typedef struct pm_batch_tuning {
   int32_t knn_warps;   /* warps per block of the persistent kNN kernel, 1..8 */
-  int32_t knn_chunk;   /* consecutive queries per warp work item, 1..1024    */
+  int32_t knn_chunk;   /* consecutive queries per warp work item, 1..1024;
+                          not read (nor tuned) when tiles answer the queries */
   int32_t knn_buffer;  /* candidate buffer per warp: 512 (k <= 224) or 2048  */
   int32_t bvh_stack;   /* BVH traversal stack entries: 16, 32 or 64          */
   int32_t block;       /* threads per block of trace and camera: 64..256     */
