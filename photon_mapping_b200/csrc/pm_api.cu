@@ -114,8 +114,9 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
 
 // A scratch buffer of `bytes` for work on stream st, ordered after the work
 // that used it last (whatever stream that was on); `done` must be recorded
-// on st once the last kernel that touches the buffer is enqueued.
-static int take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st, StreamScratch** out) {
+// on st once the last kernel that touches the buffer is enqueued. Null when
+// there is none to be had (no memory).
+static StreamScratch* take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st) {
   StreamScratch* pick = nullptr;
   for (auto& x : c->stream_scratch) {
     if (x.done && cudaEventQuery(x.done) != cudaSuccess) {
@@ -130,13 +131,13 @@ static int take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st, StreamScratch*
   cudaError_t e = cudaSuccess;
   if (!pick->done) e = cudaEventCreateWithFlags(&pick->done, cudaEventDisableTiming);
   else e = cudaStreamWaitEvent(st, pick->done, 0);
-  if (e != cudaSuccess) return cuda_status(c, e, "query scratch");
   // growing frees the old buffer, which waits for the device
-  if (pick->buf.ensure(bytes) != PM_OK)
-    return set_err(c, PM_ERR_OUT_OF_MEMORY, "query scratch (%zu bytes)", bytes);
+  if (e != cudaSuccess || pick->buf.ensure(bytes) != PM_OK) {
+    cudaGetLastError();
+    return nullptr;
+  }
   pick->last = st;
-  *out = pick;
-  return PM_OK;
+  return pick;
 }
 
 bool use_tiles(const pm_ctx* c, const DevMap& dm, int64_t nq, int k, bool sorted) {
@@ -144,14 +145,16 @@ bool use_tiles(const pm_ctx* c, const DevMap& dm, int64_t nq, int k, bool sorted
          k <= kTileMaxK && !c->stats_on;
 }
 
+// Scratch of radiance_unordered for nq queries on stream st; null without
+// memory for it, and the estimates are knn_kernel's then.
+static StreamScratch* unordered_scratch(pm_ctx* c, int64_t nq, cudaStream_t st) {
+  return take_scratch(c, 4 * (4 * (size_t)nq + sort_hist_words(nq) + 16), st);
+}
+
 // Radiance estimates of unordered device queries on stream st: their order
 // by Morton code, then the tile kernel, then what it left.
-int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq, int k,
-                       float n_emitted, float* d_rgb, cudaStream_t st) {
-  const size_t words = 4 * (size_t)nq + sort_hist_words(nq) + 16;
-  StreamScratch* sc = nullptr;
-  int s = take_scratch(c, words * 4, st, &sc);
-  if (s != PM_OK) return s;
+static int radiance_unordered(pm_ctx* c, const DevMap& dm, const void* d_q, int64_t nq, int k,
+                              float n_emitted, float* d_rgb, cudaStream_t st, StreamScratch* sc) {
   // the work counter, for one launch after the other: like the rest of the
   // buffer it is nobody else's until `done`, however many calls are in flight
   unsigned long long* counter = (unsigned long long*)sc->buf.ptr;
@@ -439,8 +442,11 @@ int pm_photonmap_radiance(pm_ctx* c, int map, const pm_radiance_query* q,
   // the tile kernel reads and writes records in another order than the
   // caller's, which host memory serves badly: queries and output are staged
   // on the device and stream through the mapping whole
-  const bool tiles = use_tiles(c, dm, nq, k, false);
-  if (tiles) d_q = mapped_out = nullptr;
+  StreamScratch* sc = nullptr;
+  if (use_tiles(c, dm, nq, k, false) && c->q_in.ensure(qb) == PM_OK &&
+      c->q_out.ensure(ob) == PM_OK)
+    sc = unordered_scratch(c, nq, st);
+  if (sc) d_q = mapped_out = nullptr;
   int s = PM_OK;
   if ((!d_q && (s = c->q_in.ensure(qb))) || (!mapped_out && (s = c->q_out.ensure(ob))))
     return set_err(c, s, "query buffers");
@@ -452,8 +458,8 @@ int pm_photonmap_radiance(pm_ctx* c, int map, const pm_radiance_query* q,
   KnnOut o{};
   o.stats = c->stats_ptr();
   o.rgb = mapped_out ? mapped_out : (float*)c->q_out.ptr;
-  if (tiles) {
-    if ((s = radiance_unordered(c, dm, d_q, nq, k, (float)n_emitted, o.rgb, st)) != PM_OK)
+  if (sc) {
+    if ((s = radiance_unordered(c, dm, d_q, nq, k, (float)n_emitted, o.rgb, st, sc)) != PM_OK)
       return s;
   } else {
     e = knn_launch(map_view(dm), d_q, nq, k, kModeRadiance,
@@ -487,11 +493,14 @@ int pm_photonmap_radiance_device(pm_ctx* c, int map, const void* d_queries,
   // a captured launch keeps no buffer of the context: it takes the
   // warp-per-query kernel, which needs none
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  StreamScratch* sc = nullptr;
   if (use_tiles(c, dm, nq, k, false) &&
       cudaStreamIsCapturing(as_stream(stream), &cap) == cudaSuccess &&
       cap == cudaStreamCaptureStatusNone)
+    sc = unordered_scratch(c, nq, as_stream(stream));
+  if (sc)
     return radiance_unordered(c, dm, d_queries, nq, k, (float)n_emitted, (float*)d_out_rgb,
-                              as_stream(stream));
+                              as_stream(stream), sc);
   KnnOut o{};
   o.stats = c->stats_ptr();
   o.rgb = (float*)d_out_rgb;

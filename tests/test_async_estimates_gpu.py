@@ -57,3 +57,56 @@ def test_more_calls_in_flight_than_the_context_has_counters(own):
     assert all(torch.equal(o, long_want) for o in long_got)
     for row in got:
         assert all(torch.equal(o, w) for o, w in zip(row, want))
+
+
+@pytest.mark.parametrize("mapped", (False, True))
+def test_estimates_without_memory_for_query_buffers(own, mapped):
+    """Little device memory left: the estimates take the kernel that needs none (with
+    page-locked host buffers, which it reads and writes in place, or device ones)."""
+    import torch
+    nq = 4_000_000
+    q = torch.from_numpy(W.wall_queries(nq, 7))
+    dq = q.cuda()
+    want = alone(own, dq)
+    fill = []
+    with Context(0) as c2:
+        pm = PhotonMap(c2)
+        pm.setPhotons(W.wall_photons(N, 1))
+        pm.build()
+        few = torch.empty((1000, 3), device="cuda")
+        call(c2, dq[:1000], few, torch.cuda.current_stream())
+        if mapped:
+            want_h = want.cpu()
+            hq, ho = q.pin_memory(), torch.empty((nq, 3)).pin_memory()
+            del dq, want
+            torch.cuda.empty_cache()
+        else:
+            got = torch.empty_like(want)
+        torch.cuda.synchronize()
+        try:
+            # all but less than the call's buffers (64 MB for the sort alone)
+            while (free := torch.cuda.mem_get_info()[0]) > 48 << 20:
+                part = max((free - (24 << 20)) & ~((2 << 20) - 1), 2 << 20)
+                while part >= 2 << 20:
+                    try:
+                        fill.append(torch.empty(part, dtype=torch.uint8, device="cuda"))
+                        break
+                    except torch.OutOfMemoryError:
+                        part //= 2
+                else:
+                    break
+            assert torch.cuda.mem_get_info()[0] < 60 << 20
+            if mapped:
+                c2.check(c2.lib.pm_photonmap_radiance(
+                    c2.handle, 0, hq.data_ptr(), nq, K, N, ho.data_ptr()),
+                    "pm_photonmap_radiance")
+            else:
+                call(c2, dq, got, torch.cuda.current_stream())
+                torch.cuda.synchronize()
+        finally:
+            fill.clear()
+            torch.cuda.empty_cache()
+        if mapped:
+            np.testing.assert_array_equal(ho.numpy(), want_h.numpy())
+        else:
+            assert torch.equal(got, want)
