@@ -141,7 +141,11 @@ int pm_photonmap_radiance(pm_ctx* ctx, int map, const pm_radiance_query* q,
                           int64_t nq, int k, int64_t n_emitted,
                           float* out_rgb);
 
-/* Same as pm_photonmap_radiance with device pointers, asynchronous. */
+/* Same as pm_photonmap_radiance with device pointers, asynchronous. A call
+ * with many queries (nq (k + 50) >= 5,000,000) uses a buffer of the context, 17
+ * bytes per query; a stream's first such call, and one with many more queries
+ * than any before, allocates it, which may wait for the device. Without memory
+ * for it, and under stream capture, the call does without, slower. */
 int pm_photonmap_radiance_device(pm_ctx* ctx, int map, const void* d_queries,
                                  int64_t nq, int k, int64_t n_emitted,
                                  void* d_out_rgb, void* stream);

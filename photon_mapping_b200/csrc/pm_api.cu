@@ -6,6 +6,7 @@
 #include "pm_knn_tile.cuh"
 #include "pm_sort.cuh"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 
@@ -117,22 +118,25 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
 // on st once the last kernel that touches the buffer is enqueued. Null when
 // there is none to be had (no memory).
 static StreamScratch* take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st) {
+  // the stream's own buffer, busy or not (its order keeps the calls apart), so
+  // that a stream with many calls in flight has one; then an idle one
   StreamScratch* pick = nullptr;
+  for (auto& x : c->stream_scratch)
+    if (!pick && x.done && x.last == st) pick = &x;
   for (auto& x : c->stream_scratch) {
-    if (x.done && cudaEventQuery(x.done) != cudaSuccess) {
-      cudaGetLastError();  // still in use
-      if (x.last == st && !pick) pick = &x;
-      continue;
-    }
-    pick = &x;
-    break;
+    if (pick) break;
+    if (!x.done || cudaEventQuery(x.done) == cudaSuccess) pick = &x;
+    else cudaGetLastError();  // still in use
   }
   if (!pick) pick = &c->stream_scratch[c->scratch_next++ % kStreamScratch];
   cudaError_t e = cudaSuccess;
   if (!pick->done) e = cudaEventCreateWithFlags(&pick->done, cudaEventDisableTiming);
   else e = cudaStreamWaitEvent(st, pick->done, 0);
-  // growing frees the old buffer, which waits for the device
-  if (e != cudaSuccess || pick->buf.ensure(bytes) != PM_OK) {
+  // growing frees the old buffer, which waits for the device: by half at least,
+  // so that a query count that creeps up seldom pays for it
+  const size_t old = pick->buf.bytes;
+  if (e != cudaSuccess || (pick->buf.ensure(bytes > old ? std::max(bytes, old + old / 2) : bytes) &&
+                           pick->buf.ensure(bytes))) {
     cudaGetLastError();
     return nullptr;
   }

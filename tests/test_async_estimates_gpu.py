@@ -110,3 +110,28 @@ def test_estimates_without_memory_for_query_buffers(own, mapped):
             np.testing.assert_array_equal(ho.numpy(), want_h.numpy())
         else:
             assert torch.equal(got, want)
+
+
+def test_calls_on_one_stream_share_a_buffer(own):
+    """Eight calls in flight on one stream, then calls that grow by 2 % each: the
+    memory taken is that of one buffer, enlarged once."""
+    import torch
+    nq = 2_000_000
+    q = torch.from_numpy(W.wall_queries(nq + nq // 3, 5)).cuda()
+    out = torch.empty((q.shape[0], 3), device="cuda")
+    st = torch.cuda.Stream()
+    call(own, q[:1000], out, st)  # kernels loaded
+    call(own, q[:MIN_QUERIES], out, st)
+    torch.cuda.synchronize()
+    free = [torch.cuda.mem_get_info()[0]]
+    for _ in range(8):
+        call(own, q[:nq], out, st)
+    torch.cuda.synchronize()
+    free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] < 2 * 17 * nq  # 16 bytes per query and the sort's table
+    for i in range(15):
+        call(own, q[:nq + nq // 50 * i], out, st)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert len(set(free[1:])) <= 2
+    torch.cuda.synchronize()
