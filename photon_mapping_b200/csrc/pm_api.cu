@@ -113,11 +113,22 @@ int build_map(pm_ctx* c, DevMap& dm, const float* d_aos, int64_t n,
   return PM_OK;
 }
 
+// Allocating, freeing and asking for an event's state are refused (and break the
+// capture) while another stream of this thread, or of any thread in the global
+// mode, is being captured, unless the thread is in the relaxed mode. Nothing
+// here goes into a capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // A scratch buffer of `bytes` for work on stream st, ordered after the work
 // that used it last (whatever stream that was on); `done` must be recorded
 // on st once the last kernel that touches the buffer is enqueued. Null when
 // there is none to be had (no memory).
 static StreamScratch* take_scratch(pm_ctx* c, size_t bytes, cudaStream_t st) {
+  const RelaxedCapture relaxed;
   // the stream's own buffer, busy or not (its order keeps the calls apart), so
   // that a stream with many calls in flight has one; then an idle one
   StreamScratch* pick = nullptr;

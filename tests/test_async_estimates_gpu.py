@@ -135,3 +135,27 @@ def test_calls_on_one_stream_share_a_buffer(own):
         free.append(torch.cuda.mem_get_info()[0])
     assert len(set(free[1:])) <= 2
     torch.cuda.synchronize()
+
+
+def test_call_beside_a_capture(own):
+    """A call on a stream that captures nothing, while another stream's capture (in
+    the global mode, the default) goes on."""
+    import torch
+    q = torch.from_numpy(W.wall_queries(MIN_QUERIES, 6)).cuda()
+    with Context(0) as c2:
+        pm = PhotonMap(c2)
+        pm.setPhotons(W.wall_photons(N, 1))
+        pm.build()
+        want = alone(c2, q)  # kernels loaded
+    x, got = torch.zeros(1, device="cuda"), torch.empty_like(want)
+    other, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        call(own, q, got, other)
+        x.add_(1)
+    g.replay()
+    torch.cuda.synchronize()
+    assert x.item() == 2
+    assert torch.equal(got, want)
+    del g
