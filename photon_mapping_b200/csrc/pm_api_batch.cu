@@ -483,7 +483,9 @@ int plan(pm_batch* b) {
       (e = cudaStreamSynchronize(b->st)))
     return bcuda(b, e, "batch plan");
   b->nq = nq;
-  b->tiles = b->max_k <= kTileMaxK && b->nq * (b->max_k + 50) >= kTileMinWork / 2;
+  bool large = false;  // a map that takes tiles
+  for (int i = 0; i < n; ++i) large |= b->stored[i] >= kTileMinPhotons;
+  b->tiles = large && b->max_k <= kTileMaxK && b->nq * (b->max_k + 50) >= kTileMinWork / 2;
   if (b->tiles && (e = batch_tile_prepare(b->max_k, &b->tile_per_sm)))
     return bcuda(b, e, "kNN set-up");
   if ((e = batch_knn_prepare(b->tune.knn_warps, b->tune.knn_buffer, &b->knn_per_sm)))

@@ -135,7 +135,8 @@ void batch_query_ranges_launch(const unsigned long long* sorted_keys, int64_t nq
 // resident blocks per SM; call it before capturing a launch in a graph.
 // left: when not null, only the queries at the sorted places left[0 .. *left_n)
 // are answered, one per work item (item_off and chunk unused), trying the squared
-// radius left_tau of each first.
+// radius left_tau of each first; a negative left_tau stands for -left_tau
+// consecutive places.
 cudaError_t batch_knn_prepare(int warps, int buffer, int* blocks_per_sm);
 cudaError_t batch_knn_launch(const BatchTables& t, const float4* slots, const uint32_t* order,
                              const int64_t* qoff, const int64_t* item_off, int64_t max_items,

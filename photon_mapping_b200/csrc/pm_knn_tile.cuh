@@ -15,7 +15,8 @@ struct TileLevels {
 // places in the sorted order), and how many.
 struct TileDefer {
   uint32_t* list;
-  float* tau;  // a squared radius to try for each of them (0: none known)
+  float* tau;  // a squared radius to try for each of them (0: none known), or minus
+               // the number of consecutive places that the entry stands for
   uint32_t* count;
   bool positions;
 };

@@ -1221,11 +1221,13 @@ __global__ void __launch_bounds__(256, 4)
       r_hint = -1.f;
     }
     const int64_t qb = left ? at : qoff[sc] + (at - ioff[sc]) * chunk;
-    const int64_t qe = left ? at + 1 : min(qoff[sc + 1], qb + chunk);
+    const float lt = left ? left_tau[c0] : 0.f;  // negative: minus the queries of the entry
+    const int64_t qe = left ? at + (lt < 0.f ? (int64_t)-lt : 1) : min(qoff[sc + 1], qb + chunk);
     // knn_chunk reads the radius of query qb, so the array starts c0 - qb away
     knn_chunk<C, kModeRadiance, false, false>(wmap[warp], wlev[warp], s, lane, slots, qb, qe, k,
                                               n_emitted, out, order, 4, r_hint, true,
-                                              left ? left_tau + (int64_t)c0 - qb : nullptr);
+                                              left && !(lt < 0.f) ? left_tau + (int64_t)c0 - qb
+                                                                  : nullptr);
   }
 }
 
