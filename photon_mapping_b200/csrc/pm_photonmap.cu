@@ -923,6 +923,10 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
           tg = r_hint > 0.f ? 1.69f * r_hint * r_hint : even_tau(m, L.oc[m.nlevels - 1].x, k);
         if (!(tg > 1e-37f)) tg = 1e-37f;  // NaN too
         q.tau = tg;
+        if (m.n <= k) {  // every photon is kept
+          guess = false;
+          q.tau = kInf;
+        }
       }
       for (int attempt = 0;; ++attempt) {
         if (need_cold) {
