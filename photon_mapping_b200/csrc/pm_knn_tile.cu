@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
 // sorted queries of one scene. A warp switches its copy of the map when the
 // scene changes. Scenes whose map is too small leave their items whole, so that
 // the warp-per-query kernel goes from neighbour to neighbour there (24 scenes of
-// 3,600 photons, 1.4M queries, k = 50: 3.41 ms before there were tiles, 4.69 ms
+// 3,600 photons, 1.4M queries, k = 50: 2.55 ms; 3.41 before there were tiles, 4.69
 // with every query left by itself). Measured on
 // 8 random scenes (50k to 1M photons emitted, k = 50 and 100): 2.63 ms for the
 // estimates of a step, 7.97 ms by the warp-per-query kernel.

@@ -262,6 +262,15 @@ static_assert(kChunk % 8 == 0 && kTail % 8 == 0, "items start at multiples of 8"
 // which matters when the output is mapped host memory.
 constexpr int kStageWords = 24;
 
+// Rounds of a loop over the buffer that are unrolled: k <= 224 has few rounds and
+// is short of instruction cache, larger k runs on 16 warps per SM and needs its
+// accesses in flight (k = 300 on 4,000 photons, 100k queries: 1.04 ms rolled, 1.02
+// unrolled).
+template <int C>
+__host__ __device__ constexpr int loop_unroll() {
+  return C <= 512 ? 1 : 4;
+}
+
 template <int C>
 struct WarpBuf {
   uint32_t key[C];  // float bits of dist2 (non-negative: order == uint order)
@@ -313,10 +322,15 @@ __device__ __forceinline__ uint32_t orig_index(const float4* pos4, uint32_t s) {
 // are skipped. Returns the value; *rank_eq = rank still needed among the
 // entries equal to it (>= 1), *n_eq = how many entries equal it.
 // Precondition: 1 <= kk <= number of valid entries.
+//
+// Its loops are not unrolled: the search is inlined with this selection at every
+// place that may need it, and what a query executes has to stay in the
+// instruction cache (knn_chunk).
 template <class Get>
 __device__ uint32_t warp_select(uint32_t* hist, int cnt, uint32_t kk, Get get,
                                 int lane, uint32_t* rank_eq, uint32_t* n_eq) {
   uint32_t vor = 0, vand = 0xffffffffu, nvalid = 0;
+#pragma unroll 1
   for (int i = lane; i < cnt; i += 32) {
     uint32_t v;
     if (get(i, v)) {
@@ -343,6 +357,7 @@ __device__ uint32_t warp_select(uint32_t* hist, int cnt, uint32_t kk, Get get,
   for (; shift >= 0; shift -= 8) {
     for (int b = lane; b < 256; b += 32) hist[b] = 0;
     __syncwarp();
+#pragma unroll 1
     for (int i = lane; i < cnt; i += 32) {
       uint32_t v;
       if (get(i, v) && (v & pmask) == prefix)
@@ -458,6 +473,7 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
   if (!(tau > 0.f) || !(sc < __int_as_float(0x7f800000))) return false;
   for (int b = lane; b < 256; b += 32) s.hist[b] = 0;
   __syncwarp();
+#pragma unroll (loop_unroll<C>())
   for (int i = lane; i < cnt; i += 32) {
     const float d2 = __uint_as_float(s.key[i]);
     const int b = min(255, __float2int_rz(__fmul_rz(d2, sc)));
@@ -468,6 +484,7 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
   const int bin = (int)hist_find(s.hist, (uint32_t)k, lane, &kk, &nb);
   if (nb > 32) return false;
   int at = 0;
+#pragma unroll (loop_unroll<C>())
   for (int base = 0; base < cnt; base += 32) {
     const int i = base + lane;
     bool in = false;
@@ -548,6 +565,7 @@ __device__ __forceinline__ int compact_kept(const float4* pos4, WarpBuf<C>& s,
                                             int cnt, uint32_t kth_key,
                                             uint32_t kth_oid, int lane) {
   int dst = 0;
+#pragma unroll (loop_unroll<C>())
   for (int b = 0; b < cnt; b += 32) {
     const int i = b + lane;
     const bool v = i < cnt;
@@ -574,28 +592,34 @@ __device__ __forceinline__ int compact_kept(const float4* pos4, WarpBuf<C>& s,
 // in a fixed tree, so the sum depends on the kept photons alone: the tile
 // kernel (pm_knn_tile.cu) adds in the same order. The photons of each class
 // are queued in s.key (its distances are no longer needed), C / 32 per class;
-// should a class need more, its lane reads the whole list instead.
+// should a class need more, its lane reads the whole list instead. Without
+// `classes` (maps and k that tiles never answer) lane l takes entries l, l + 32, ..
+// of the list, which is in the walk's order whatever the radius was.
 template <int C>
 __device__ __forceinline__ float3 kept_sum(const MapDev& m, WarpBuf<C>& s, int nk, float3 ns,
-                                           int lane) {
+                                           int lane, bool classes) {
   constexpr int kRows = C / 32;
-  uint32_t* const queue = s.key;
-  uint32_t* const count = s.hist;
-  count[lane] = 0;
-  __syncwarp();
-  for (int b = 0; b < nk; b += 32) {
-    const bool in = b + lane < nk;
-    const uint32_t id = in ? s.id[b + lane] : 0u;
-    const uint32_t c = in ? id & 31u : 32u;
-    const unsigned peers = __match_any_sync(kFull, c);
-    const uint32_t before = in ? count[c] : 0u;
-    const uint32_t r = before + __popc(peers & lt_mask(lane));
+  uint32_t* const queue = classes ? s.key : s.id;
+  int n = (nk - lane + 31) >> 5;
+  if (classes) {
+    uint32_t* const count = s.hist;
+    count[lane] = 0;
     __syncwarp();
-    if (in && r < kRows) queue[r * 32 + c] = id;
-    if (in && (peers >> lane) == 1u) count[c] = r + 1;  // the class's last peer
-    __syncwarp();
+#pragma unroll 1
+    for (int b = 0; b < nk; b += 32) {
+      const bool in = b + lane < nk;
+      const uint32_t id = in ? s.id[b + lane] : 0u;
+      const uint32_t c = in ? id & 31u : 32u;
+      const unsigned peers = __match_any_sync(kFull, c);
+      const uint32_t before = in ? count[c] : 0u;
+      const uint32_t r = before + __popc(peers & lt_mask(lane));
+      __syncwarp();
+      if (in && r < kRows) queue[r * 32 + c] = id;
+      if (in && (peers >> lane) == 1u) count[c] = r + 1;  // the class's last peer
+      __syncwarp();
+    }
+    n = (int)count[lane];
   }
-  const int n = (int)count[lane];
   float x = 0.f, y = 0.f, z = 0.f;
   auto add = [&](uint32_t id) {
     const float4 t = __ldg(m.thr4 + id);
@@ -607,8 +631,10 @@ __device__ __forceinline__ float3 kept_sum(const MapDev& m, WarpBuf<C>& s, int n
     }
   };
   if (n <= kRows) {
+#pragma unroll 2
     for (int r = 0; r < n; ++r) add(queue[r * 32 + lane]);
   } else {
+#pragma unroll 1
     for (int i = 0; i < nk; ++i)
       if ((s.id[i] & 31u) == (uint32_t)lane) add(s.id[i]);
   }
@@ -643,8 +669,26 @@ __device__ __forceinline__ uint2 tighten(const float4* pos4, WarpBuf<C>* sp,
   return make_uint2((uint32_t)n2, kth_key);
 }
 
-// Appends photon i (position p) when valid and dist2 <= tau. When the
-// buffer is nearly full, keeps the k best and lowers tau to the k-th.
+// When the buffer may lack room for `room` more entries, keeps the k best and lowers
+// tau to the k-th.
+template <int C, bool S>
+__device__ __forceinline__ void cut(const MapDev& m, Query& q, WarpBuf<C>& s, int lane, int room) {
+  if (q.cnt > C - room - kStageWords) {
+    __syncwarp();
+    const uint2 r = tighten<C, S>(m.pos4, &s, q.cnt, q.k, q.tau, lane);
+    q.cnt = (int)r.x;
+    q.tau = __uint_as_float(r.y);
+  }
+}
+
+// A small buffer is cut after two appends, which halves the copies of the cut in
+// the code; a large one after each.
+template <int C>
+__host__ __device__ constexpr bool cut_by_two() {
+  return C <= 512;
+}
+
+// Appends photon i (position p) when valid and dist2 <= tau.
 template <int C, bool S>
 __device__ __forceinline__ void offer(const MapDev& m, Query& q, WarpBuf<C>& s,
                                       int lane, const float4& p, int i,
@@ -658,12 +702,7 @@ __device__ __forceinline__ void offer(const MapDev& m, Query& q, WarpBuf<C>& s,
     s.id[o] = (uint32_t)i;
   }
   q.cnt += __popc(bal);
-  if (q.cnt > C - 32 - kStageWords) {
-    __syncwarp();
-    const uint2 r = tighten<C, S>(m.pos4, &s, q.cnt, q.k, q.tau, lane);
-    q.cnt = (int)r.x;
-    q.tau = __uint_as_float(r.y);
-  }
+  if (!cut_by_two<C>()) cut<C, S>(m, q, s, lane, 32);
 }
 
 // Scans the photons of the ng groups listed in s.list: lane l handles
@@ -685,6 +724,7 @@ __device__ __forceinline__ void scan_groups(const MapDev& m, Query& q,
     const float4 pb = __ldg(m.pos4 + (vb ? ib : 0));
     offer<C, S>(m, q, s, lane, pa, ia, va);
     if (r + 4 < ng) offer<C, S>(m, q, s, lane, pb, ib, vb);
+    if (cut_by_two<C>()) cut<C, S>(m, q, s, lane, 64);
   }
   __syncwarp();
 }
@@ -701,6 +741,7 @@ __device__ __forceinline__ void scan_range(const MapDev& m, Query& q,
     const float4 pb = __ldg(m.pos4 + (vb ? ib : lo));
     offer<C, S>(m, q, s, lane, pa, ia, va);
     if (b + 32 < hi) offer<C, S>(m, q, s, lane, pb, ib, vb);
+    if (cut_by_two<C>()) cut<C, S>(m, q, s, lane, 64);
   }
 }
 
@@ -828,6 +869,13 @@ __device__ __forceinline__ float cold_tau(const float4* pos4, const float4* boxe
 }
 
 // Answers queries [qb, qe) of a work item on map m, one at a time (one warp).
+// Bound by issue, and by the instruction cache where a query is short: the code of
+// a query with the sums by class, unrolled loops and a cut at each append no
+// longer fitted (3.2 warps per issue waited for instructions, 0.6 before those
+// sums): 1M sorted queries of 3,000 photons, k = 50, took 2.22 instead of 1.62 ms,
+// of 30 photons 2.06 instead of 0.75; 1.55 and 0.56 with the loops rolled, fewer
+// copies of the cut, sums by class only where tiles need them and no guesses for
+// maps of k photons or fewer.
 // r_hint: the last exact k-th distance this warp found (in/out).
 // HIO (the single-map kernel, whose queries and output may be mapped host
 // memory): radiance records are prefetched one query ahead with cp.async,
@@ -1003,7 +1051,8 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       const float4 r2 = HIO ? s.rec[buf][2] : __ldg(q4 + 2);
       const float cos_o = dot_ref(r1.x, r1.y, r1.z, r2.x, r2.y, r2.z);
       const int nk = all ? cnt : compact_kept(m.pos4, s, cnt, kth_key, kth_oid, lane);
-      const float3 sum = kept_sum(m, s, nk, make_float3(r2.x, r2.y, r2.z), lane);
+      const float3 sum = kept_sum(m, s, nk, make_float3(r2.x, r2.y, r2.z), lane,
+                                  m.n >= kTileMinPhotons && k <= kTileMaxK);
       if (lane < 3) {  // a lane per channel
         const float o = kept > 0 ? radiance_from_sum(lane == 0 ? sum.x : lane == 1 ? sum.y : sum.z,
                                                      lane == 0 ? r0.w : lane == 1 ? r1.w : r2.w,
