@@ -400,7 +400,8 @@ __global__ void widen_kernel(const float4* __restrict__ binary, int n, float4* _
   w[5] = make_float4(hi[0].z, hi[1].z, hi[2].z, hi[3].z);
   w[6] = make_float4(__int_as_float(id[0]), __int_as_float(id[1]), __int_as_float(id[2]),
                      __int_as_float(id[3]));
-  w[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int left = __float_as_int(b0.w);
+  w[7] = make_float4(__int_as_float(left < 0 ? 1 : 2), b0.w, b1.w, 0.f);
 }
 
 static float host_from_ordered(uint32_t u) {

@@ -12,7 +12,8 @@
 //                      up to 4 grandchildren (a child that is a leaf counts
 //                      itself): lo.x, lo.y, lo.z, hi.x, hi.y, hi.z of the four,
 //                      their ids (>= 0: inner node, < 0: leaf ~id, kNoChild:
-//                      none), and 16 bytes of padding to a 128-byte line. A walk
+//                      none), and {entries of the left child (1: a leaf, or 2),
+//                      left child, right child, -} of the binary node. A walk
 //                      from node 0 takes two levels of the binary tree per step.
 #pragma once
 
@@ -63,19 +64,30 @@ __device__ __forceinline__ bool ray_triangle(V3 o, V3 d, V3 p0, V3 e1, V3 e2,
 
 constexpr int kNoChild = (int)0x80000000;
 
-// Entries of the traversal stack of a walk that the binary tree would give
-// STACK: a step pushes up to 3 where two levels of the binary tree push 2. (16
-// gives 23: a tree of equal boxes that needs 17 of the binary walk is to be
-// refused there, as it always was.)
+// Entries of the stack of a walk for which STACK was chosen. A step pushes up to 3
+// where two levels of the binary tree push 2. With 32 and 64 that holds any tree a
+// mesh gives (17 full levels need 2^34 faces); a ray that needs more sets error bit 0.
+// 16 can be too few, and no ratio of the two walks' needs holds for every tree, so a
+// ray that finds the smaller stack full is answered by the binary walk
+// (intersect_binary) and 16 accepts whatever that does with 16 entries. (One entry
+// less than 3 per 2: full trees of one level more, the first that the binary walk
+// refuses, fill 24.) Walks for 32 and 64 leave the binary walk out: with the call in
+// it the path tracer took 3.97 ms instead of 3.65 (512 x 512 x 4, 563k faces).
+template <int STACK>
+__host__ __device__ constexpr bool stack_refers() {
+  return STACK <= 16;
+}
 template <int STACK>
 __host__ __device__ constexpr int stack_entries() {
-  return STACK + STACK / 2 - (STACK == 16 ? 1 : 0);
+  return STACK + STACK / 2 - (stack_refers<STACK>() ? 1 : 0);
 }
+constexpr int kStackFull = -2;  // the "next node" of a ray for the binary walk
 
 // One step of a walk: the boxes of node `node` against the ray (o, inv) in
 // [tmin, tmax]. Returns the inner child entered first (-1: none) and pushes the
-// other inner children hit, the nearest on top; `leaves` gets a bit per leaf
-// child hit, its id in ids.
+// other inner children hit, the nearest on top; when they do not fit, the walk is
+// over with kStackFull (REFERS), or they are lost and error bit 0 is set. `leaves`
+// gets a bit per leaf child hit, its id in ids.
 //
 // Slab test; NaN products (0 * inf) impose no constraint. The exit distance is
 // widened by 1 + 2*gamma(3) (Ize 2013) and the boxes themselves are padded at
@@ -102,7 +114,7 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   return r;
 }
 
-template <int N>
+template <bool REFERS, int N>
 __device__ __forceinline__ int walk_step(const float4* __restrict__ nodes, int node,
                                          const RayPacked& r, float tmin, float tmax,
                                          int (&stack)[N], int& sp, int* err, unsigned& leaves,
@@ -156,6 +168,7 @@ __device__ __forceinline__ int walk_step(const float4* __restrict__ nodes, int n
     if (more > 2) stack[sp] = child(key[3]);
     sp += more;
   } else {
+    if (REFERS) return kStackFull;
     atomicOr(err, 1);  // their subtrees are lost
   }
   if (key[0] != 0xffffffffu) return child(key[0]);
@@ -180,9 +193,70 @@ __device__ __forceinline__ void test_leaf(const SceneDev& sc, int leaf, V3 o,
   }
 }
 
+// intersect_t by the binary tree, from the same records: a binary child's box is that
+// of its own children. For the few rays that need more stack than a walk has;
+// one that needs more than STACK entries here sets error bit 0 and loses the
+// subtree.
+template <int STACK>
+__device__ __noinline__ Hit intersect_binary(const float4* __restrict__ nodes,
+                                             const float4* __restrict__ mt, int* err, V3 o, V3 d,
+                                             float tmin, float tmax) {
+  SceneDev sc{};
+  sc.mt = mt;
+  Hit h{tmax, 0.f, 0.f, -1};
+  const V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+  // entry distance into the box of entries [a, b) of node n, if it is met (the
+  // arithmetic of walk_step)
+  auto enter = [&](const float* n, int a, int b, float& tn) {
+    float lo[3], hi[3];
+    for (int x = 0; x < 3; ++x) {
+      lo[x] = n[4 * x + a];
+      hi[x] = n[12 + 4 * x + a];
+      for (int e = a + 1; e < b; ++e) {
+        lo[x] = fminf(lo[x], n[4 * x + e]);
+        hi[x] = fmaxf(hi[x], n[12 + 4 * x + e]);
+      }
+    }
+    const float x0 = (lo[0] - o.x) * inv.x, x1 = (hi[0] - o.x) * inv.x;
+    const float y0 = (lo[1] - o.y) * inv.y, y1 = (hi[1] - o.y) * inv.y;
+    const float z0 = (lo[2] - o.z) * inv.z, z1 = (hi[2] - o.z) * inv.z;
+    tn = fmaxf(fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fminf(z0, z1)), tmin);
+    const float tf = fminf(fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1)), h.t);
+    return tn <= tf * 1.00000072f;
+  };
+  int stack[STACK];
+  int sp = 0;
+  int node = 0;
+  while (true) {
+    const float* n = reinterpret_cast<const float*>(nodes + 8 * (size_t)node);
+    const int nl = __float_as_int(n[28]);
+    const int left = __float_as_int(n[29]), right = __float_as_int(n[30]);
+    float tl, tr;
+    const bool hl = enter(n, 0, nl, tl);
+    const bool hr = enter(n, nl, nl + (right < 0 ? 1 : 2), tr);
+    if (hl && left < 0) test_leaf(sc, ~left, o, d, tmin, h);
+    if (hr && right < 0) test_leaf(sc, ~right, o, d, tmin, h);
+    int next = hl && left >= 0 ? left : -1;
+    if (hr && right >= 0) {
+      int other = next;
+      if (next < 0 || tr < tl) next = right;
+      else other = right;
+      if (other >= 0) {
+        if (sp < STACK) stack[sp++] = other;
+        else atomicOr(err, 1);
+      }
+    }
+    if (next < 0) {
+      if (sp == 0) return h;
+      next = stack[--sp];
+    }
+    node = next;
+  }
+}
+
 // Closest hit with tmin <= t <= tmax; ties in t go to the smaller face id,
-// so the result does not depend on the traversal order. STACK entries of
-// traversal stack (an overflow sets error bit 0 and loses the subtree).
+// so the result does not depend on the traversal order. STACK: entries of
+// traversal stack (stack_entries).
 template <int STACK>
 __device__ __forceinline__ bool intersect_t(const SceneDev& sc, V3 o, V3 d,
                                             float tmin, float tmax, Hit& h) {
@@ -202,7 +276,8 @@ __device__ __forceinline__ bool intersect_t(const SceneDev& sc, V3 o, V3 d,
   while (node >= 0) {
     unsigned leaves;
     int4 ids;
-    node = walk_step(sc.nodes, node, r, tmin, h.t, stack, sp, sc.err, leaves, ids);
+    node = walk_step<stack_refers<STACK>()>(sc.nodes, node, r, tmin, h.t, stack, sp, sc.err,
+                                            leaves, ids);
     while (leaves) {
       const int i = __ffs(leaves) - 1;
       leaves &= leaves - 1;
@@ -210,6 +285,10 @@ __device__ __forceinline__ bool intersect_t(const SceneDev& sc, V3 o, V3 d,
       const int id = i & 2 ? hi : lo;
       if (id != kNoChild) test_leaf(sc, ~id, o, d, tmin, h);
     }
+  }
+  if constexpr (stack_refers<STACK>()) {
+    if (node == kStackFull)
+      h = intersect_binary<STACK>(sc.nodes, sc.mt, sc.err, o, d, tmin, tmax);
   }
   return h.prim >= 0;
 }
@@ -235,7 +314,7 @@ struct Walk {
   RayPacked r;
   float tmin;
   Hit h;
-  int node;  // inner node to visit next, -1: none
+  int node;  // inner node to visit next, -1: none, kStackFull: h is not to be had here
   int sp;
   int waiting;  // leaves in the queue
 
@@ -260,11 +339,11 @@ struct Walk {
   }
 
   // Visits `node`; can_visit() holds.
-  template <int BLOCK, int N>
+  template <int BLOCK, bool REFERS, int N>
   __device__ __forceinline__ void visit(int (&stack)[N], int* queue, int* err) {
     unsigned leaves;
     int4 ids;
-    node = walk_step(nodes, node, r, tmin, h.t, stack, sp, err, leaves, ids);
+    node = walk_step<REFERS>(nodes, node, r, tmin, h.t, stack, sp, err, leaves, ids);
     const int id[4] = {ids.x, ids.y, ids.z, ids.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i)

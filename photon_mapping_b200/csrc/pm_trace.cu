@@ -256,6 +256,12 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
     bool leave = false;  // the lane has a vertex to go on from
     if (state == kHit) {
       const TraceArgs& a = args(src);
+      if constexpr (stack_refers<STACK>()) {
+        const SceneDev& sc = scene(src);
+        if (w.node == kStackFull)
+          w.h = intersect_binary<STACK>(sc.nodes, sc.mt, sc.err, p.org, p.dir, kRayEps,
+                                        __int_as_float(0x7f7fffff));
+      }
       leave = photon_hit<MODE>(scene(src), a, p, w.h, rs, v);
       if (!leave) {
         if (MODE != kTraceReplay && a.store_count) a.store_count[g] = (uint32_t)p.nst;
@@ -308,7 +314,8 @@ __device__ __forceinline__ void trace_persistent(unsigned long long* next, long 
       if (__popc(leaf) >= __popc(inner)) {  // a walking lane is in one of them: never both empty
         if (state == kWalk && w.waiting > 0) w.test<BLOCK>(p.org, p.dir, queue);
       } else {
-        if (state == kWalk && w.can_visit()) w.visit<BLOCK>(stack, queue, scene(src).err);
+        if (state == kWalk && w.can_visit())
+          w.visit<BLOCK, stack_refers<STACK>()>(stack, queue, scene(src).err);
       }
     }
   }
