@@ -55,6 +55,7 @@ __device__ __forceinline__ void emit_query(const RenderArgs& a, int64_t base,
 template <int STACK>
 __device__ V3 direct_light(const SceneDev& sc, const Surf& s, V3 wo,
                            const Material& m, Rng& rng) {
+  if (sc.n_lights == 0) return v3(0.f, 0.f, 0.f);  // no light to sample
   float pc, pp;
   const int lf = sample_light(sc, rng, pc);
   Surf ls;
