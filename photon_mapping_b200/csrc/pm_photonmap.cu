@@ -262,13 +262,14 @@ static_assert(kChunk % 8 == 0 && kTail % 8 == 0, "items start at multiples of 8"
 // which matters when the output is mapped host memory.
 constexpr int kStageWords = 24;
 
-// Rounds of a loop over the buffer that are unrolled: k <= 224 has few rounds and
-// is short of instruction cache, larger k runs on 16 warps per SM and needs its
-// accesses in flight (k = 300 on 4,000 photons, 100k queries: 1.04 ms rolled, 1.02
-// unrolled).
-template <int C>
-__host__ __device__ constexpr int loop_unroll() {
-  return C <= 512 ? 1 : 4;
+// Whether loops over the buffer are rolled and the buffer is cut after two appends
+// instead of each (half the copies of the cut in the code): estimates with k <= 224.
+// Larger k runs on 16 warps per SM and needs its accesses in flight (k = 300 on 4,000
+// photons, 100k queries: 1.04 ms rolled, 1.02 unrolled), and neighbour lists have no
+// sums to make room for (64 queries: 66.8 us rolled, 65.0 unrolled).
+template <int C, int MODE>
+__host__ __device__ constexpr bool rolled() {
+  return C <= 512 && MODE != kModeKnn;
 }
 
 template <int C>
@@ -323,14 +324,14 @@ __device__ __forceinline__ uint32_t orig_index(const float4* pos4, uint32_t s) {
 // entries equal to it (>= 1), *n_eq = how many entries equal it.
 // Precondition: 1 <= kk <= number of valid entries.
 //
-// Its loops are not unrolled: the search is inlined with this selection at every
-// place that may need it, and what a query executes has to stay in the
-// instruction cache (knn_chunk).
-template <class Get>
+// For estimates its loops are not unrolled: the search is inlined with this
+// selection at every place that may need it, and what a query executes has to stay
+// in the instruction cache (knn_chunk).
+template <int MODE, class Get>
 __device__ uint32_t warp_select(uint32_t* hist, int cnt, uint32_t kk, Get get,
                                 int lane, uint32_t* rank_eq, uint32_t* n_eq) {
   uint32_t vor = 0, vand = 0xffffffffu, nvalid = 0;
-#pragma unroll 1
+#pragma unroll (MODE == kModeKnn ? 4 : 1)
   for (int i = lane; i < cnt; i += 32) {
     uint32_t v;
     if (get(i, v)) {
@@ -357,7 +358,7 @@ __device__ uint32_t warp_select(uint32_t* hist, int cnt, uint32_t kk, Get get,
   for (; shift >= 0; shift -= 8) {
     for (int b = lane; b < 256; b += 32) hist[b] = 0;
     __syncwarp();
-#pragma unroll 1
+#pragma unroll (MODE == kModeKnn ? 4 : 1)
     for (int i = lane; i < cnt; i += 32) {
       uint32_t v;
       if (get(i, v) && (v & pmask) == prefix)
@@ -463,7 +464,7 @@ __device__ __forceinline__ uint32_t hist_find(const uint32_t* hist, uint32_t kk,
 // critical bin holds one or two entries. Returns false (caller falls back
 // to the radix select) when tau is not a positive finite bound or the
 // critical bin holds more than 32 entries.
-template <int C>
+template <int C, int MODE>
 __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
                                                 WarpBuf<C>& s, int cnt, int k,
                                                 float tau, int lane,
@@ -473,7 +474,7 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
   if (!(tau > 0.f) || !(sc < __int_as_float(0x7f800000))) return false;
   for (int b = lane; b < 256; b += 32) s.hist[b] = 0;
   __syncwarp();
-#pragma unroll (loop_unroll<C>())
+#pragma unroll (rolled<C, MODE>() ? 1 : 4)
   for (int i = lane; i < cnt; i += 32) {
     const float d2 = __uint_as_float(s.key[i]);
     const int b = min(255, __float2int_rz(__fmul_rz(d2, sc)));
@@ -484,7 +485,7 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
   const int bin = (int)hist_find(s.hist, (uint32_t)k, lane, &kk, &nb);
   if (nb > 32) return false;
   int at = 0;
-#pragma unroll (loop_unroll<C>())
+#pragma unroll (rolled<C, MODE>() ? 1 : 4)
   for (int base = 0; base < cnt; base += 32) {
     const int i = base + lane;
     bool in = false;
@@ -522,15 +523,15 @@ __device__ __forceinline__ bool select_kth_hist(const float4* pos4,
 // Exact k-th smallest (dist2, index) pair of the buffer: kth_key, and
 // kth_oid = largest original index kept among entries with key == kth_key
 // (0xffffffff when all of them are kept). Every entry has dist2 <= tau.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void select_kth(const float4* pos4, WarpBuf<C>& s,
                                            int cnt, int k, float tau, int lane,
                                            uint32_t& kth_key,
                                            uint32_t& kth_oid) {
   uint32_t rank_eq, n_eq;
   stat_add<S>(s, lane, kStatSelects, 1);
-  if (select_kth_hist(pos4, s, cnt, k, tau, lane, kth_key, kth_oid)) return;
-  kth_key = warp_select(
+  if (select_kth_hist<C, MODE>(pos4, s, cnt, k, tau, lane, kth_key, kth_oid)) return;
+  kth_key = warp_select<MODE>(
       s.hist, cnt, (uint32_t)k,
       [&](int i, uint32_t& v) {
         v = s.key[i];
@@ -541,7 +542,7 @@ __device__ __forceinline__ void select_kth(const float4* pos4, WarpBuf<C>& s,
   if (rank_eq != n_eq) {
     uint32_t r2, n2;
     const uint32_t kk = kth_key;
-    kth_oid = warp_select(
+    kth_oid = warp_select<MODE>(
         s.hist, cnt, rank_eq,
         [&](int i, uint32_t& v) {
           if (s.key[i] != kk) return false;
@@ -560,12 +561,12 @@ __device__ __forceinline__ bool keep_entry(const float4* pos4, uint32_t key,
   return kth_oid == 0xffffffffu || orig_index(pos4, id) <= kth_oid;
 }
 
-template <int C>
+template <int C, int MODE>
 __device__ __forceinline__ int compact_kept(const float4* pos4, WarpBuf<C>& s,
                                             int cnt, uint32_t kth_key,
                                             uint32_t kth_oid, int lane) {
   int dst = 0;
-#pragma unroll (loop_unroll<C>())
+#pragma unroll (rolled<C, MODE>() ? 1 : 4)
   for (int b = 0; b < cnt; b += 32) {
     const int i = b + lane;
     const bool v = i < cnt;
@@ -659,37 +660,30 @@ struct Query {
 
 // Rare path, kept out of line: the buffer is nearly full. Keeps the k best
 // entries; returns {new count, float bits of the k-th distance}.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ uint2 tighten(const float4* pos4, WarpBuf<C>* sp,
                                          int cnt, int k, float tau, int lane) {
   WarpBuf<C>& s = *sp;
   uint32_t kth_key, kth_oid;
-  select_kth<C, S>(pos4, s, cnt, k, tau, lane, kth_key, kth_oid);
-  const int n2 = compact_kept(pos4, s, cnt, kth_key, kth_oid, lane);
+  select_kth<C, MODE, S>(pos4, s, cnt, k, tau, lane, kth_key, kth_oid);
+  const int n2 = compact_kept<C, MODE>(pos4, s, cnt, kth_key, kth_oid, lane);
   return make_uint2((uint32_t)n2, kth_key);
 }
 
 // When the buffer may lack room for `room` more entries, keeps the k best and lowers
 // tau to the k-th.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void cut(const MapDev& m, Query& q, WarpBuf<C>& s, int lane, int room) {
   if (q.cnt > C - room - kStageWords) {
     __syncwarp();
-    const uint2 r = tighten<C, S>(m.pos4, &s, q.cnt, q.k, q.tau, lane);
+    const uint2 r = tighten<C, MODE, S>(m.pos4, &s, q.cnt, q.k, q.tau, lane);
     q.cnt = (int)r.x;
     q.tau = __uint_as_float(r.y);
   }
 }
 
-// A small buffer is cut after two appends, which halves the copies of the cut in
-// the code; a large one after each.
-template <int C>
-__host__ __device__ constexpr bool cut_by_two() {
-  return C <= 512;
-}
-
 // Appends photon i (position p) when valid and dist2 <= tau.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void offer(const MapDev& m, Query& q, WarpBuf<C>& s,
                                       int lane, const float4& p, int i,
                                       bool valid) {
@@ -702,13 +696,13 @@ __device__ __forceinline__ void offer(const MapDev& m, Query& q, WarpBuf<C>& s,
     s.id[o] = (uint32_t)i;
   }
   q.cnt += __popc(bal);
-  if (!cut_by_two<C>()) cut<C, S>(m, q, s, lane, 32);
+  if (!rolled<C, MODE>()) cut<C, MODE, S>(m, q, s, lane, 32);
 }
 
 // Scans the photons of the ng groups listed in s.list: lane l handles
 // photon (l & 7) of group 4r + (l >> 3) in round r; two rounds are loaded
 // before either is used.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void scan_groups(const MapDev& m, Query& q,
                                             WarpBuf<C>& s, int lane, int ng) {
   const int sub = lane >> 3, j = lane & 7;
@@ -722,15 +716,15 @@ __device__ __forceinline__ void scan_groups(const MapDev& m, Query& q,
     const bool va = ga < ng && ia < m.n, vb = gb < ng && ib < m.n;
     const float4 pa = __ldg(m.pos4 + (va ? ia : 0));
     const float4 pb = __ldg(m.pos4 + (vb ? ib : 0));
-    offer<C, S>(m, q, s, lane, pa, ia, va);
-    if (r + 4 < ng) offer<C, S>(m, q, s, lane, pb, ib, vb);
-    if (cut_by_two<C>()) cut<C, S>(m, q, s, lane, 64);
+    offer<C, MODE, S>(m, q, s, lane, pa, ia, va);
+    if (r + 4 < ng) offer<C, MODE, S>(m, q, s, lane, pb, ib, vb);
+    if (rolled<C, MODE>()) cut<C, MODE, S>(m, q, s, lane, 64);
   }
   __syncwarp();
 }
 
 // Scans the contiguous photon range [lo, hi), 32 photons per round.
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void scan_range(const MapDev& m, Query& q,
                                            WarpBuf<C>& s, int lane, int lo,
                                            int hi) {
@@ -739,9 +733,9 @@ __device__ __forceinline__ void scan_range(const MapDev& m, Query& q,
     const bool va = ia < hi, vb = ib < hi;
     const float4 pa = __ldg(m.pos4 + (va ? ia : lo));
     const float4 pb = __ldg(m.pos4 + (vb ? ib : lo));
-    offer<C, S>(m, q, s, lane, pa, ia, va);
-    if (b + 32 < hi) offer<C, S>(m, q, s, lane, pb, ib, vb);
-    if (cut_by_two<C>()) cut<C, S>(m, q, s, lane, 64);
+    offer<C, MODE, S>(m, q, s, lane, pa, ia, va);
+    if (b + 32 < hi) offer<C, MODE, S>(m, q, s, lane, pb, ib, vb);
+    if (rolled<C, MODE>()) cut<C, MODE, S>(m, q, s, lane, 64);
   }
 }
 
@@ -752,13 +746,13 @@ __device__ __forceinline__ void scan_range(const MapDev& m, Query& q,
 // candidate appends and the rare buffer cut, and a second copy of it made
 // the kernel 1.9 % slower (3.387 against 3.324 ms on 1M primary-hit queries
 // at k = 100; same scan order, same results).
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ void collect(const MapDev& m, const Levels& L,
                                         Query& q, WarpBuf<C>& s, int lane) {
   q.cnt = 0;
   stat_add<S>(s, lane, kStatWalks, 1);
   if (m.nlevels == 1) {  // a single 8-photon group
-    scan_range<C, S>(m, q, s, lane, 0, m.n);
+    scan_range<C, MODE, S>(m, q, s, lane, 0, m.n);
     return;
   }
   if (lane == 0) s.stack[0] = ((uint32_t)(m.nlevels - 1) << 28);
@@ -794,7 +788,7 @@ __device__ __forceinline__ void collect(const MapDev& m, const Levels& L,
     // full rounds of 8 groups after a bottom-level node, the rest at the end
     const int take = done ? pending : (cl == 0 ? (pending & ~7) : 0);
     if (take > 0) {
-      scan_groups<C, S>(m, q, s, lane, take);
+      scan_groups<C, MODE, S>(m, q, s, lane, take);
       const int rest = pending - take;
       uint32_t keep = 0;
       if (lane < rest) keep = s.list[take + lane];
@@ -821,7 +815,7 @@ __device__ __forceinline__ unsigned long long warp_min_u64(
 // greedily (nearest box at each level), then take the k-th distance among
 // the photons of the Morton-adjacent groups around it (real photons, so
 // the bound holds).
-template <int C, bool S>
+template <int C, int MODE, bool S>
 __device__ __forceinline__ float cold_tau(const float4* pos4, const float4* boxes,
                                        int n, int nlevels, const Levels* Lp,
                                        float qx, float qy, float qz, int k,
@@ -857,14 +851,14 @@ __device__ __forceinline__ float cold_tau(const float4* pos4, const float4* boxe
   const int want = min(ngroups, max(32, (k + kGroup - 1) / kGroup + 8));
   const int first =
       max(0, min(want == 32 ? (node & ~31) : node - want / 2, ngroups - want));
-  scan_range<C, S>(m, q, s, lane, first * kGroup, min(n, (first + want) * kGroup));
+  scan_range<C, MODE, S>(m, q, s, lane, first * kGroup, min(n, (first + want) * kGroup));
   __syncwarp();
   if (q.cnt < k) return __int_as_float(0x7f800000);
   uint32_t mx = 0;
   for (int i = lane; i < q.cnt; i += 32) mx = max(mx, s.key[i]);
   mx = __reduce_max_sync(kFull, mx);  // every entry lies in [0, mx]
   uint32_t kth_key, kth_oid;
-  select_kth<C, S>(pos4, s, q.cnt, k, __uint_as_float(mx), lane, kth_key, kth_oid);
+  select_kth<C, MODE, S>(pos4, s, q.cnt, k, __uint_as_float(mx), lane, kth_key, kth_oid);
   return __uint_as_float(kth_key);
 }
 
@@ -978,12 +972,12 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       }
       for (int attempt = 0;; ++attempt) {
         if (need_cold) {
-          q.tau = cold_tau<C, S>(m.pos4, m.boxes, m.n, m.nlevels, &L, q.x, q.y,
+          q.tau = cold_tau<C, MODE, S>(m.pos4, m.boxes, m.n, m.nlevels, &L, q.x, q.y,
                                  q.z, k, &s, lane);
           need_cold = false;
           guess = false;
         }
-        collect<C, S>(m, L, q, s, lane);
+        collect<C, MODE, S>(m, L, q, s, lane);
         if (warm_guess) {
           if (q.cnt >= k) break;
           warm_guess = false;
@@ -1013,7 +1007,7 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       for (int i = lane; i < cnt; i += 32) mx = max(mx, s.key[i]);
       kth_key = __reduce_max_sync(kFull, mx);
     } else {
-      select_kth<C, S>(m.pos4, s, cnt, k, q.tau, lane, kth_key, kth_oid);
+      select_kth<C, MODE, S>(m.pos4, s, cnt, k, q.tau, lane, kth_key, kth_oid);
     }
     const int kept = all ? cnt : k;
     const float maxd2 = kept > 0 ? __uint_as_float(kth_key) : 0.f;
@@ -1027,7 +1021,7 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       const float4 r2 = HIO ? s.rec[buf][2] : __ldg(q4 + 2);
       const float ax = out.adj_in[3 * rec], ay = out.adj_in[3 * rec + 1],
                   az = out.adj_in[3 * rec + 2];
-      const int nk = all ? cnt : compact_kept(m.pos4, s, cnt, kth_key, kth_oid, lane);
+      const int nk = all ? cnt : compact_kept<C, MODE>(m.pos4, s, cnt, kth_key, kth_oid, lane);
       if (kept > 0 && (ax != 0.f || ay != 0.f || az != 0.f)) {
         const float cos_o = dot_ref(r1.x, r1.y, r1.z, r2.x, r2.y, r2.z);
         const float den = __fmul_rn(__fmul_rn(n_emitted, kPI), maxd2);
@@ -1050,7 +1044,7 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       const float4 r1 = HIO ? s.rec[buf][1] : __ldg(q4 + 1);
       const float4 r2 = HIO ? s.rec[buf][2] : __ldg(q4 + 2);
       const float cos_o = dot_ref(r1.x, r1.y, r1.z, r2.x, r2.y, r2.z);
-      const int nk = all ? cnt : compact_kept(m.pos4, s, cnt, kth_key, kth_oid, lane);
+      const int nk = all ? cnt : compact_kept<C, MODE>(m.pos4, s, cnt, kth_key, kth_oid, lane);
       const float3 sum = kept_sum(m, s, nk, make_float3(r2.x, r2.y, r2.z), lane,
                                   m.n >= kTileMinPhotons && k <= kTileMaxK);
       if (lane < 3) {  // a lane per channel
@@ -1080,7 +1074,7 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
       }
     } else {
       int n2 = cnt;
-      if (!all) n2 = compact_kept(m.pos4, s, cnt, kth_key, kth_oid, lane);
+      if (!all) n2 = compact_kept<C, MODE>(m.pos4, s, cnt, kth_key, kth_oid, lane);
       for (int i = lane; i < n2; i += 32)
         s.id[i] = orig_index(m.pos4, s.id[i]);
       __syncwarp();
