@@ -37,3 +37,26 @@ def test_tiles_answer_one_about_as_fast_as_two(ctx):
             t.append(a.elapsed_time(b))
         ms[k] = min(t)
     assert ms[1] < 4 * ms[2], ms
+
+
+@pytest.mark.parametrize("n", (5000, 100_000, 1_000_000))
+def test_one_scans_no_more_than_four(ctx, n):
+    """Photon groups scanned per neighbour list, by the kernel's own counters: the
+    nearest photon needs no more of them than the four nearest (68 against 9 in 1M
+    photons when the radius crept up and the search fell back to the patch bound)."""
+    pm = PhotonMap(ctx)
+    pm.setPhotons(W.wall_photons(n, 1))
+    pm.build()
+    q = np.ascontiguousarray(W.wall_queries(20_000, 2)[:, :3])
+    per = {}
+    for k in (1, 4):
+        ctx.get_stats(reset=True)
+        ctx.set_stats(True)
+        try:
+            pm.query_knn(q, k)
+        finally:
+            ctx.set_stats(False)
+        st = ctx.get_stats(reset=True)
+        assert st["queries"] == len(q)
+        per[k] = st["leaves"] / st["queries"]
+    assert per[1] <= per[4], per
