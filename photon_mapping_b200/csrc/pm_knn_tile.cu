@@ -57,6 +57,18 @@ constexpr float kNextSlack = 1.15f;
 constexpr float kWalkReach = 25.f;
 constexpr float kSubReach = 4.f;
 constexpr int kTries = 24;
+// When a warp stops trying. Where photons crowd the tree's sort cells, groups overlap
+// so much that a list fills at any radius, or the radius that a query needs meets too
+// many: with 24 tries for every item, 150k estimates on 500k clustered photons (k =
+// 50) took 10.1 ms, and on photons with a few far outside three times as long as
+// by the warp-per-query kernel; 2.8 ms and its time this way.
+// Walks of one query that may find too many groups, each at a quarter of the
+// radius, before the queries are left; and in a warp whose last item was left so.
+constexpr int kFullWalks = 4;
+constexpr int kFullWalksWary = 1;
+// Queries are left once a radius with too few photons is this part of one with too
+// many groups: in between, one or the other would come again.
+constexpr float kNoRoom = 0.2f;
 
 struct TileWarp {
   uint32_t list[4][kListCap];
@@ -67,6 +79,14 @@ struct TileWarp {
   uint32_t ccnt[kSubQ], kth[kSubQ];
   uint32_t key[kSubQ][kCrit], oid[kSubQ][kCrit];  // photons around the k-th
   uint16_t at[kSubQ][kCrit];                      // and their bytes' places
+  // Of the first query left: the largest squared radius known to hold fewer than k
+  // photons, the smallest known to meet too many groups, and the walks that did.
+  // Every lane writes and reads the same value (registers are short).
+  float few, many;
+  int full;
+  // The warp's last item was left without an answer, as the next will be where groups
+  // overlap too much for lists: a query by itself finds out.
+  int wary;
 };
 
 // Words of one query's bytes ([row / 4][lane], 4 rows per word); 4 more keep the
@@ -311,11 +331,18 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
   if (!A && lane < nq && bad) rgb[3 * (size_t)rec] = rgb[3 * (size_t)rec + 1] = rgb[3 * (size_t)rec + 2] = 0.f;
   unsigned todo = __ballot_sync(kFull, lane < nq && !bad);
   float good = tau;      // from the last queries answered
-  int span = kTileQ, sq = kSubQ, tries = 0;
+  int span = s.wary ? 1 : kTileQ, sq = kSubQ, tries = 0;
+  s.few = 0.f;
+  s.many = FLT_MAX;
+  s.full = 0;
   while (todo) {
     const float tw = tau * kWalkSlack;
-    if (++tries > kTries || !(tw > 1e-30f && tw < 1e30f)) {
-      if ((todo >> lane) & 1u) leave(defer, defer.positions ? (uint32_t)(q0 + lane) : rec, tau);
+    const bool hopeless = s.few >= kNoRoom * s.many ||
+                          s.full > (s.wary ? kFullWalksWary : kFullWalks);
+    if (__any_sync(kFull, ++tries > kTries || !(tw > 1e-30f && tw < 1e30f) || hopeless)) {
+      const float hint = s.few > 0.f ? 2.f * s.few : s.full > 0 ? 0.f : tau;
+      if ((todo >> lane) & 1u) leave(defer, defer.positions ? (uint32_t)(q0 + lane) : rec, hint);
+      s.wary = 1;
       break;
     }
     unsigned wm = near_run(todo, span, kWalkReach * tau, px, py, pz, lane);
@@ -323,8 +350,16 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
         tile_walk(m, L, s, stack, warp_box(px, py, pz, (wm >> lane) & 1u), tw, lane);
     if (mine < 0) {
       // too many groups: the queries lie apart, or the radius is too large
-      if (__popc(wm) > 1) span = max(1, __popc(wm) >> 1);
-      else tau *= 0.25f;
+      if (__popc(wm) > 1) {
+        span = max(1, __popc(wm) >> 1);
+      } else {
+        const int full = s.full;
+        __syncwarp();
+        s.full = full + 1;
+        s.many = fminf(s.many, tau);
+        tau *= 0.25f;
+        __syncwarp();
+      }
       continue;
     }
     float tf = tau;
@@ -335,9 +370,13 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
       const int used =
           tile_filter(m, none, s, sub, rows, mine, warp_box(px, py, pz, in), tf, lane);
       if (used > rows) {
-        if (sq > 1) sq >>= 1;
-        else tf *= 0.5f;
-        if (++tries > kTries) break;
+        if (ns > 1) {
+          sq = ns >> 1;
+        } else {
+          s.many = fminf(s.many, tf);
+          tf *= 0.5f;
+        }
+        if (++tries > kTries || s.few >= kNoRoom * s.many) break;
         continue;
       }
       // the sub-tile's queries in order; absent ones are NaN
@@ -442,7 +481,8 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
         float need = 0.f;
         if (fail) need = tf * (chi > 0 ? fminf(1.2f * (float)k / (float)chi, 4.f) : 4.f);
         need = fmaxf(redux_max(need), 1.1f * tf);
-        if (++tries > kTries) break;
+        if (ns == 1) s.few = fmaxf(s.few, tf);
+        if (++tries > kTries || s.few >= kNoRoom * s.many) break;
         tau = need;
         tf = need;
         if (need > tw) break;  // walk again
@@ -668,7 +708,10 @@ __device__ __forceinline__ void tile_item(const MapDev& m, const TileLevels& L, 
       if (far != 0u) good = tau = kNextSlack * __uint_as_float(far);
       tf = fminf(tau, tw);
       tries = 0;
-      if (sq < kSubQ) sq <<= 1;
+      s.few = 0.f;
+      s.many = FLT_MAX;
+      s.full = s.wary = 0;
+      sq = min(2 * sq, kSubQ);
       __syncwarp();
     }
     if (span < kTileQ && !wm) span <<= 1;
@@ -716,6 +759,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
   }
   __syncthreads();
   float tau = even_tau(m, L.oc[m.nlevels - 1].x, k);
+  s.wary = 0;
   while (true) {
     unsigned long long c0 = 0;
     if (lane == 0) c0 = atomicAdd(counter, 1ull);
@@ -753,6 +797,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
   const int64_t total = ioff[t.n_scenes];
   int cur = -1, k = 0;
   float tau = 0.f, n_emitted = 0.f;
+  s.wary = 0;
   while (true) {
     unsigned long long c0 = 0;
     if (lane == 0) c0 = atomicAdd(counter, 1ull);
@@ -766,6 +811,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 5)
       if (lane < kMaxLevels) wlev[warp].oc[lane] = make_int2(bs.map.lvl_off[lane], bs.map.lvl_cnt[lane]);
       __syncwarp();
       cur = sc;
+      s.wary = 0;
       k = bs.k;
       n_emitted = bs.n_emitted;
       if (wmap[warp].n >= kTileMinPhotons)
