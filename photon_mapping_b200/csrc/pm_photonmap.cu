@@ -985,12 +985,13 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
           continue;
         }
         if (!guess || q.cnt >= k) break;
-        if (attempt < 4) {
-          // on surfaces the count grows about as the squared radius; without any
-          // photon it may be anything (1M queries of 3M photons, k = 1: 9.5 ms at
-          // 1.4 k times, 3.26 at 4, 3.08 at 8, 2.62 at 16, which is slower in a volume)
-          const float grow = fminf(1.4f * (float)k / (float)max(q.cnt, 1), 16.f);
-          tg *= q.cnt > 0 ? grow : fmaxf(grow, 8.f);
+        if (attempt < 6) {
+          // on surfaces the count grows about as the squared radius; no more than
+          // fourfold, as queries off the surfaces meet a crowd behind an empty
+          // stretch (300k queries off 500k clustered photons, k = 200: 6.02 ms grown
+          // up to 16-fold, 4.09 so), and fourfold without any photon (1M queries of 3M
+          // photons, k = 1: 9.5 ms at 1.4 k, 3.17 so)
+          tg *= q.cnt > 0 ? fmaxf(2.f, fminf(1.4f * (float)k / (float)q.cnt, 4.f)) : 4.f;
           q.tau = tg;
         } else {
           need_cold = true;

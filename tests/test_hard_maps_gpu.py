@@ -81,3 +81,23 @@ def test_tiles_on_hard_maps(ctx, kind, off, n, nq, k, slower):
     ctx.get_stats(reset=True)
     np.testing.assert_array_equal(out[0].cpu().numpy(), out[1].cpu().numpy())
     assert slower is None or ms[0] < slower * ms[1], ms
+
+
+def test_radius_off_the_surfaces_does_not_overshoot(ctx):
+    """Photon groups scanned per neighbour list at points off clustered photons, by the
+    kernel's own counters: 1,459 when a radius grew up to 16-fold, 982 since it grows
+    fourfold at most."""
+    n, k = 500_000, 200
+    ph = photons_of("clusters", n)
+    pm = PhotonMap(ctx)
+    pm.setPhotons(ph)
+    pm.build()
+    q = queries_of(ph, 20_000, True)
+    ctx.get_stats(reset=True)
+    ctx.set_stats(True)
+    try:
+        pm.query_knn(np.ascontiguousarray(q[:, :3]), k)
+    finally:
+        ctx.set_stats(False)
+    st = ctx.get_stats(reset=True)
+    assert st["leaves"] < 1200 * st["queries"], st
