@@ -986,12 +986,14 @@ __device__ __forceinline__ void knn_chunk(const MapDev& m, const Levels& L, Warp
         }
         if (!guess || q.cnt >= k) break;
         if (attempt < 6) {
-          // on surfaces the count grows about as the squared radius; no more than
-          // fourfold, as queries off the surfaces meet a crowd behind an empty
-          // stretch (300k queries off 500k clustered photons, k = 200: 6.02 ms grown
-          // up to 16-fold, 4.09 so), and fourfold without any photon (1M queries of 3M
-          // photons, k = 1: 9.5 ms at 1.4 k, 3.17 so)
-          tg *= q.cnt > 0 ? fmaxf(2.f, fminf(1.4f * (float)k / (float)q.cnt, 4.f)) : 4.f;
+          // on surfaces the count grows about as the squared radius. From another
+          // query's radius no more than fourfold, as queries off the surfaces meet a
+          // crowd behind an empty stretch (300k queries off 500k clustered photons, k =
+          // 200: 6.02 ms grown up to 16-fold, 4.09 so), and fourfold without any
+          // photon (1M queries of 3M photons, k = 1: 9.5 ms at 1.4 k, 3.17 so). A warp's
+          // first query has farther to go (64 lists, a warp each: 68.2 us at fourfold, 65.0)
+          const float most = r_hint > 0.f ? 4.f : 16.f;
+          tg *= q.cnt > 0 ? fminf(1.4f * (float)k / (float)q.cnt, most) : most;
           q.tau = tg;
         } else {
           need_cold = true;
