@@ -708,6 +708,8 @@ def run_ours(args) -> None:
         "gpu_launches": args.steps * LAUNCHES_PER_STEP,
         "parity": parity,
         "knn_per_query": per_q,
+        # statistics select the warp-per-query kernel; the timed steps run the tiles
+        "knn_per_query_kernel": "knn_kernel (not the tile kernel of the timed steps)",
         "knn_uniform_cube": uniform,
         "photon_trace": {"emitted": N_EMIT, "stored": trace_stats["stored"],
                          "seconds": trace_s, "photons_per_s": N_EMIT / trace_s,

@@ -71,8 +71,9 @@ const char* pm_ctx_last_error(const pm_ctx* ctx);
 /* Static name of a status code. */
 const char* pm_status_string(int status);
 
-/* Counters of the k-nearest-neighbour kernels (diagnostics; no reference
- * counterpart). Collected only while enabled with pm_ctx_set_stats. */
+/* Counters of the warp-per-query kernel (diagnostics; no reference
+ * counterpart). Collected only while enabled with pm_ctx_set_stats, and every
+ * query takes that kernel then, also those that tiles would answer. */
 typedef struct pm_knn_stats {
   uint64_t queries;     /* queries answered                                  */
   uint64_t cold_starts; /* queries whose search radius was bounded afresh    */

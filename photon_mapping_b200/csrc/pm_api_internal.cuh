@@ -120,9 +120,12 @@ struct StreamScratch {
 
 // Least work, as queries x (k + 50), for which tiles of sorted queries are used:
 // below, the sort and the latency of a tile cost more than the warp-per-query
-// kernel. Measured with unordered queries on maps of 50k to 1M photons: both
-// take the same time at 70k queries for k = 10, 60k for 50, 33k for 100 and 16k
-// for 300. Queries sorted anyway (renders) need half.
+// kernel. Set with unordered queries on maps of 50k to 1M photons, where both took
+// the same time at 70k queries for k = 10, 60k for 50, 33k for 100 and 16k for 300.
+// With the warp-per-query kernel as it is now, tiles against it at the line, us: k =
+// 10 169 / 197 (50k photons) and 287 / 243 (1M), k = 50 158 / 175 and 217 / 209, k =
+// 100 141 / 132 and 207 / 153, k = 300 179 / 330 and 271 / 352; at twice the work 196 /
+// 272 to 242 / 284 for k = 50 and 100. Queries sorted anyway (renders) need half.
 constexpr int64_t kTileMinWork = 5000000;
 
 }  // namespace pm

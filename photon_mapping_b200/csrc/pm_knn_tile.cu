@@ -53,7 +53,9 @@ constexpr int kFewEnough = 8;   // ... that end the search for the k-th
 constexpr float kWalkSlack = 1.6f;
 constexpr float kNextSlack = 1.15f;
 // Largest distance (squared, over the search radius squared) from the first
-// query of a walk, or of a sub-tile, to its others.
+// query of a walk, or of a sub-tile, to its others. Frames and 65k to 900k unordered
+// queries: a walk's 9 is the same within 1 %, 100 up to 2.5 % slower; a sub-tile's 1 is
+// 2 to 12 % slower, 16 up to 4 %.
 constexpr float kWalkReach = 25.f;
 constexpr float kSubReach = 4.f;
 constexpr int kTries = 24;

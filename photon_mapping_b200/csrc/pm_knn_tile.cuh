@@ -39,6 +39,8 @@ constexpr int kQueryKeyBits = 24;
 void query_keys_launch(const MapDev& m, const void* queries, int64_t nq, int stride4,
                        uint32_t* keys, uint32_t* vals, cudaStream_t st);
 
+// No crossing: tiles are faster from 1,000 photons on (1M queries, k = 50: 0.59 against
+// 1.57 ms; 100k: 0.15 against 0.19). The size from which the tests cover them.
 constexpr int kTileMinPhotons = 4096;
 constexpr int kTileMaxK = 448;
 // With photon_adj, the adjoint instead (KnnOut::adj_in, photon_adj; rgb unused).

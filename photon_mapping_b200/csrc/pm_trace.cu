@@ -393,7 +393,8 @@ static int trace_pace(int64_t paths) {
 void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int stack,
                         cudaStream_t st) {
   if (total_emit <= 0) return;
-  // persistent: as many blocks as fit at once (2048 threads per SM)
+  // persistent: blocks for 2048 threads per SM. The launch bounds make 768 of them
+  // resident at once; blocks that start later find the indices spent and end
   const long long cap = (long long)sm_count() * (2048 / block);
   const unsigned gb = (unsigned)std::min<long long>(cap, (total_emit + block - 1) / block);
   cudaMemsetAsync(t.next_photon, 0, sizeof(unsigned long long), st);
@@ -409,7 +410,8 @@ void batch_trace_launch(const BatchTables& t, int64_t total_emit, int block, int
 void trace_launch(const SceneDev& sc, const TraceArgs& a, cudaStream_t st) {
   if (a.n_emit <= 0) return;
   const int tb = kTraceBlock;
-  // persistent: as many blocks as fit at once (2048 threads per SM)
+  // persistent: blocks for 2048 threads per SM. The launch bounds make 768 of them
+  // resident at once; blocks that start later find the indices spent and end
   const long long cap = (long long)sm_count() * (2048 / tb);
   const int gb = (int)std::min<long long>(cap, (a.n_emit + tb - 1) / tb);
   cudaMemsetAsync(a.next, 0, sizeof(unsigned long long), st);
